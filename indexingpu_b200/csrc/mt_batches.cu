@@ -24,7 +24,7 @@
 
 #include <algorithm>
 
-#include "mt_internal.cuh"
+#include "mt_lane.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -140,7 +140,7 @@ template <int T, int OP>
 __global__ void __launch_bounds__(kBlock, min_blocks_for<OP>) batches_class_kernel(tree_view tv, batches_view b,
                                                                                      uint32_t sb) {
   if (b.status[0]) return;
-  constexpr uint32_t cls = OP == OP_FIND ? 0u : (OP == OP_PASS_INSERT ? 1u : 2u);
+  constexpr uint32_t cls = OP == OP_PASS_INSERT ? 1u : 2u;
   tile<T> t;
   const uint32_t tile_id = (blockIdx.x * blockDim.x + threadIdx.x) / T;
   const uint32_t num_tiles = (gridDim.x * blockDim.x) / T;
@@ -150,11 +150,23 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for<OP>) batches_class_kern
   cache.release(t, tv.pool);
 }
 
+__global__ void __launch_bounds__(kBlock, MT_LANE_FIND_BLOCKS) batches_find_kernel(tree_view tv, batches_view b,
+                                                                                   uint32_t sb) {
+  if (b.status[0]) return;
+  lane_find<true>(tv, class_args(b, sb, 0u));
+}
+
 }  // namespace mtb
 
 using namespace mtb;
 
 namespace {
+
+// The sub-batches' sizes are on the device only: the grid fills the GPU.
+int launch_class_finds(mt_masstree* t, const batches_view& b, uint32_t sb, cudaStream_t s) {
+  batches_find_kernel<<<host_lane_grid(t, (const void*)batches_find_kernel, b.max_total), kBlock, 0, s>>>(t->tv, b, sb);
+  return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
+}
 
 template <int T, int OP>
 int launch_class(mt_masstree* t, const batches_view& b, uint32_t sb, cudaStream_t s) {
@@ -185,7 +197,7 @@ int launch_forked(mt_masstree* t, const batches_view& b, cudaStream_t s) {
     int rc = host_fork(t, s);
     if (rc) return rc;
     rc = launch_class_tile<OP_PASS_INSERT>(t, tw, b, sb, s);
-    if (!rc) rc = launch_class_tile<OP_FIND>(t, t->tile_size, b, sb, t->side[0]);
+    if (!rc) rc = launch_class_finds(t, b, sb, t->side[0]);
     if (!rc) rc = launch_class_tile<OP_PASS_UPDERASE>(t, tu, b, sb, t->side[1]);
     rc = host_join(t, s, rc);
     if (rc) return rc;

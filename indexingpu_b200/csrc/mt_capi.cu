@@ -21,7 +21,7 @@
 #include <unordered_map>
 #include <vector>
 
-#include "mt_internal.cuh"
+#include "mt_lane.cuh"
 
 namespace mtb {
 
@@ -157,6 +157,11 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for<OP>) batch_kernel(tree_
   cache.init(tv.pool, tile_id);
   serve_requests<T, OP, CONC>(t, tv, cache, a, tile_id, num_tiles);
   cache.release(t, tv.pool);
+}
+
+template <bool CONC>
+__global__ void __launch_bounds__(kBlock, MT_LANE_FIND_BLOCKS) find_kernel(tree_view tv, batch_args a) {
+  lane_find<CONC>(tv, a);
 }
 
 template <int T, bool CONC>
@@ -350,6 +355,18 @@ int grid_for(const mt_masstree* t, const void* fn) {
   return b * t->sms;
 }
 
+}  // namespace
+
+namespace mtb {
+int host_lane_grid(const mt_masstree* t, const void* fn, uint32_t n) {
+  const uint32_t warps_per_block = kBlock / 32;
+  const uint32_t need = n / warps_per_block + (n % warps_per_block != 0u);
+  return (int)std::max(1u, std::min<uint32_t>((uint32_t)grid_for(t, fn), need));
+}
+}  // namespace mtb
+
+namespace {
+
 int cuda_status(cudaError_t e) { return e == cudaSuccess ? MT_OK : MT_ERR_CUDA; }
 
 int launch_reclaim(mt_masstree* t, cudaStream_t s) {
@@ -380,7 +397,16 @@ int launch_batch(mt_masstree* t, const batch_args& a, cudaStream_t s) {
   if (a.n == 0) return MT_OK;
   int rc = launch_reclaim(t, s);
   if (rc) return rc;
-  return launch_batch_tile<OP, CONC>(t, OP == OP_FIND ? t->tile_size : t->write_tile_size, a, s);
+  return launch_batch_tile<OP, CONC>(t, t->write_tile_size, a, s);
+}
+
+// Finds take no slabs, so no reclaim pass precedes them.  a.n: the number of
+// requests, or (with an index) its upper bound.
+template <bool CONC>
+int launch_find(mt_masstree* t, const batch_args& a, cudaStream_t s) {
+  if (a.n == 0) return MT_OK;
+  find_kernel<CONC><<<host_lane_grid(t, (const void*)find_kernel<CONC>, a.n), kBlock, 0, s>>>(t->tv, a);
+  return cuda_status(cudaGetLastError());
 }
 
 // Slots of the update-combining table for n requests: a power of two of at
@@ -465,7 +491,7 @@ int launch_mixed_split(mt_masstree* t, batch_args a, bool bucket_keys, cudaStrea
   const uint32_t tw = t->write_tile_size <= 16 ? 16u : 32u;
   const uint32_t tu = t->upderase_tile_size ? t->upderase_tile_size : tw;
   rc = launch_batch_tile<OP_PASS_INSERT, true>(t, tw, i, s);
-  if (!rc) rc = launch_batch_tile<OP_FIND, true>(t, t->tile_size, f, t->side[0]);
+  if (!rc) rc = launch_find<true>(t, f, t->side[0]);
   if (!rc) rc = launch_combine(t, u, a.n, t->side[1]);
   if (!rc) rc = launch_batch_tile<OP_PASS_UPDERASE, true>(t, tu, u, t->side[1]);
   if (!rc) rc = launch_combine_results(t, u, a.n, t->side[1]);
@@ -672,7 +698,7 @@ int mt_find(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_t*
   a.keys = keys; a.key_lengths = klens; a.values = values; a.value_lengths_out = vlens;
   a.max_key_length = maxK; a.max_value_length = values ? maxV : 0u; a.n = n;
   cudaStream_t s = (cudaStream_t)stream;
-  return (flags & MT_FLAG_CONCURRENT) ? launch_batch<OP_FIND, true>(t, a, s) : launch_batch<OP_FIND, false>(t, a, s);
+  return (flags & MT_FLAG_CONCURRENT) ? launch_find<true>(t, a, s) : launch_find<false>(t, a, s);
 }
 
 int mt_insert(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_t* klens, const uint32_t* values,
@@ -1118,7 +1144,7 @@ extern "C" int mt_mixed_batch_noalloc(mt_masstree* t, const uint8_t* types, cons
   batch_args f = a;
   f.index = find_idx;
   f.n_dev = counts;
-  rc = launch_batch_tile<OP_MIXED, true>(t, t->tile_size, f, s);
+  rc = launch_find<true>(t, f, s);
   if (rc) return rc;
   batch_args w = a;
   w.index = write_idx;

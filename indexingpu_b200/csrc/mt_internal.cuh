@@ -19,6 +19,9 @@ constexpr uint32_t kClassBarrierMin = 1u << 17;
 #ifndef MT_MIN_BLOCKS_PER_SM
 #define MT_MIN_BLOCKS_PER_SM 8  // occupancy hint for the batch kernels: caps registers at 64
 #endif
+#ifndef MT_LANE_FIND_BLOCKS
+#define MT_LANE_FIND_BLOCKS 6  // occupancy hint for the find kernels (one request per thread)
+#endif
 #ifndef MT_WRITE_MIN_BLOCKS_PER_SM
 #define MT_WRITE_MIN_BLOCKS_PER_SM MT_MIN_BLOCKS_PER_SM  // the same for kernels that insert
 #endif
@@ -251,6 +254,7 @@ int host_merge_begin(mt_masstree* t, cudaStream_t s, uint32_t flags);
 int host_merge_end(mt_masstree* t, cudaStream_t s, int rc);
 // Host helpers implemented in mt_capi.cu.
 int host_max_blocks_per_sm(const void* fn, int block, size_t smem);
+int host_lane_grid(const mt_masstree* t, const void* fn, uint32_t n);  // blocks for n requests, one per thread
 int host_launch_reclaim(mt_masstree* t, cudaStream_t s);
 int host_fork(mt_masstree* t, cudaStream_t s);
 int host_join(mt_masstree* t, cudaStream_t s, int rc);
