@@ -50,8 +50,9 @@ enum { MT_REQ_INSERT = 0, MT_REQ_ERASE = 1, MT_REQ_FIND = 2, MT_REQ_UPDATE = 3 }
 #define MT_FLAG_USE_UPPER_KEY 4u    /* scan stops after upper_keys (reference `use_upper_key`) */
 #define MT_FLAG_SINGLE_PASS 8u      /* mixed_batch: one kernel for every kind instead of
                                        finds-then-writes passes (comparison switch) */
-#define MT_FLAG_BUCKET_KEYS 16u     /* mixed_batch(es): serve short keys before long keys in
-                                       every request class */
+#define MT_FLAG_BUCKET_KEYS 16u     /* mixed_batches: serve short keys before long keys in
+                                       every request class (accepted by mixed_batch, which
+                                       serves its requests without classes) */
 #define MT_FLAG_PERSISTENT 32u      /* mixed_batches: one cooperative persistent launch for all
                                        sub-batches instead of three class kernels per sub-batch */
 #define MT_FLAG_MERGE 64u           /* erase, mixed_batch: after the call's erases, fold nodes
@@ -92,7 +93,7 @@ typedef struct mt_stats_t {
   uint64_t total_slabs;     /* slabs in the pool (128 bytes each) */
   uint64_t used_slabs;      /* handed out and not yet returned */
   uint64_t free_slabs;      /* never used or returned */
-  uint64_t limbo_slabs;     /* retired, returned at the next call on the tree */
+  uint64_t limbo_slabs;     /* retired, returned at the next call on the tree that is not a find */
   uint32_t num_shards;
   uint32_t tile_size;
   uint32_t device_error;    /* first device error since the last mt_sync */

@@ -383,7 +383,6 @@ int host_bulk_insert(mt_masstree* t, const batch_args& a, bool upsert, cudaStrea
     // The rest through the ordinary insert kernel.
     batch_args r = a;
     r.index = b.rest;
-    r.n_dev = b.ctl + 2;
     r.n = h[2];
     rc = host_launch_insert(t, r, upsert, s);
   }

@@ -52,42 +52,6 @@ __global__ void partition_kernel(const uint8_t* types, uint32_t n, uint32_t* fin
   }
 }
 
-// Split a mixed batch into finds, inserts and updates+erases (one atomic per
-// warp and counter).  Each class has an index region of n entries; with
-// bucketing, keys longer than half the maximum length fill it from the back,
-// so that the tiles of a warp serve keys of similar length (similar paths)
-// side by side.  counts[2c] / counts[2c+1] = entries from the front / back of
-// class c's region (c = finds, inserts, updates+erases).
-__global__ void partition3_kernel(const uint8_t* types, const uint32_t* key_lengths, uint32_t max_key_length,
-                                  uint32_t bucket_keys, uint32_t n, uint32_t* find_idx, uint32_t* insert_idx,
-                                  uint32_t* upderase_idx, uint32_t* counts) {
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n;
-       base += gridDim.x * blockDim.x) {
-    const uint32_t i = base + lane;
-    const bool valid = i < n;
-    const uint32_t k = valid ? types[i] : 0xFFu;
-    const uint32_t c = k == MT_REQ_FIND ? 0u : (k == MT_REQ_INSERT ? 1u : 2u);
-    uint32_t bucket = 0;
-    if (valid && bucket_keys && key_lengths) bucket = (2u * key_lengths[i] > max_key_length) ? 1u : 0u;
-    const uint32_t slot = valid ? c * 2u + bucket : 0xFFu;
-    uint32_t m[6], b[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) m[q] = __ballot_sync(0xFFFFFFFFu, slot == (uint32_t)q);
-    if (lane == 0) {
-#pragma unroll
-      for (int q = 0; q < 6; ++q) b[q] = m[q] ? atomicAdd(counts + q, (uint32_t)__popc(m[q])) : 0u;
-    }
-#pragma unroll
-    for (int q = 0; q < 6; ++q) b[q] = __shfl_sync(0xFFFFFFFFu, b[q], 0);
-    if (valid) {
-      const uint32_t r = reg_select(b, slot) + __popc(reg_select(m, slot) & ((1u << lane) - 1u));
-      uint32_t* dst = c == 0 ? find_idx : (c == 1 ? insert_idx : upderase_idx);
-      dst[bucket ? n - 1u - r : r] = i;
-    }
-  }
-}
-
 // Update combining.  Updates of one key in one call have no order among each
 // other, so all but one of them can be linearised right before the one that
 // runs, and report its result: the final value is one of theirs either way.
@@ -162,6 +126,13 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for<OP>) batch_kernel(tree_
 template <bool CONC>
 __global__ void __launch_bounds__(kBlock, MT_LANE_FIND_BLOCKS) find_kernel(tree_view tv, batch_args a) {
   lane_find<CONC>(tv, a);
+}
+
+// Inserts, updates, erases and mixed batches, one request per lane.  4M-key
+// and 16M-key trees: see lane_serve.
+template <int OP>
+__global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) lane_kernel(tree_view tv, batch_args a, defer_list dl) {
+  lane_serve<OP>(tv, a, dl);
 }
 
 template <int T, bool CONC>
@@ -254,8 +225,10 @@ __global__ void line_atomicity_kernel(uint32_t* lines, uint32_t nlines, uint32_t
   }
 }
 
-// Return slabs retired by earlier launches to their shard's free stack.
-__global__ void reclaim_kernel(pool_view p) {
+// Return slabs retired by earlier launches to their shard's free stack, and
+// start the call's defer list (may be null) empty.
+__global__ void reclaim_kernel(pool_view p, uint32_t* defer_count) {
+  if (blockIdx.x == 0 && threadIdx.x == 0 && defer_count != nullptr) *defer_count = 0u;
   for (uint32_t s = blockIdx.x; s < p.num_shards; s += gridDim.x) {
     __shared__ int top, n;
     if (threadIdx.x == 0) {
@@ -316,7 +289,7 @@ int host_join(mt_masstree* t, cudaStream_t s, int rc) {
 }
 
 int host_launch_reclaim(mt_masstree* t, cudaStream_t s) {
-  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool);
+  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->defer_mem);
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
 }
 }  // namespace mtb
@@ -370,7 +343,7 @@ namespace {
 int cuda_status(cudaError_t e) { return e == cudaSuccess ? MT_OK : MT_ERR_CUDA; }
 
 int launch_reclaim(mt_masstree* t, cudaStream_t s) {
-  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool);
+  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->defer_mem);
   return cuda_status(cudaGetLastError());
 }
 
@@ -392,12 +365,31 @@ int launch_batch_tile(mt_masstree* t, uint32_t tile, const batch_args& a, cudaSt
   }
 }
 
-template <int OP, bool CONC>
-int launch_batch(mt_masstree* t, const batch_args& a, cudaStream_t s) {
+// Writes and mixed batches: the lane kernel, then a tile kernel for the
+// requests it hands on (few: splits of roots and full parents, new layers,
+// nodes under contention), in pieces that fit the defer list.
+template <int OP>
+int launch_lane(mt_masstree* t, batch_args a, uint32_t tile, cudaStream_t s) {
   if (a.n == 0) return MT_OK;
   int rc = launch_reclaim(t, s);
-  if (rc) return rc;
-  return launch_batch_tile<OP, CONC>(t, t->write_tile_size, a, s);
+  const defer_list dl{t->defer_mem + 32, t->defer_mem};
+  const uint32_t n = a.n;
+  for (uint32_t first = 0; !rc && first < n; first += a.n) {
+    a.first = first;
+    a.n = std::min(n - first, t->defer_cap);
+    if (first && cudaMemsetAsync(dl.count, 0, sizeof(uint32_t), s) != cudaSuccess) return MT_ERR_CUDA;
+    lane_kernel<OP><<<host_lane_grid(t, (const void*)lane_kernel<OP>, a.n), kBlock, 0, s>>>(t->tv, a, dl);
+    if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
+    batch_args d = a;
+    d.index = dl.list;
+    d.n_dev = dl.count;
+    rc = launch_batch_tile<OP, true>(t, tile, d, s);
+  }
+  return rc;
+}
+template <int OP>
+int launch_lane(mt_masstree* t, const batch_args& a, cudaStream_t s) {
+  return launch_lane<OP>(t, a, t->write_tile_size, s);
 }
 
 // Finds take no slabs, so no reclaim pass precedes them.  a.n: the number of
@@ -409,6 +401,13 @@ int launch_find(mt_masstree* t, const batch_args& a, cudaStream_t s) {
   return cuda_status(cudaGetLastError());
 }
 
+// MT_FLAG_SINGLE_PASS: one tile kernel for every kind.
+int launch_single_pass(mt_masstree* t, const batch_args& a, cudaStream_t s) {
+  if (a.n == 0) return MT_OK;
+  const int rc = launch_reclaim(t, s);
+  return rc ? rc : launch_batch_tile<OP_MIXED, true>(t, t->write_tile_size, a, s);
+}
+
 // Slots of the update-combining table for n requests: a power of two of at
 // least 2n (load factor at most one half).
 uint32_t combine_slots(uint32_t n) {
@@ -417,33 +416,30 @@ uint32_t combine_slots(uint32_t n) {
   return p;
 }
 
-// Index scratch for split mixed batches (grown on demand, kept).
-int ensure_split_scratch(mt_masstree* t, uint32_t n, cudaStream_t s) {
-  if (n <= t->split_cap) return MT_OK;
+// Combining scratch for n requests (grown on demand, kept): the table of
+// combine_slots(n) words, then leader_of (n words).
+int ensure_combine_scratch(mt_masstree* t, uint32_t n, cudaStream_t s) {
+  if (n <= t->combine_cap) return MT_OK;
   if (cudaStreamSynchronize(s) != cudaSuccess) return MT_ERR_CUDA;
-  if (t->split_idx) cudaFree(t->split_idx);
-  t->split_idx = nullptr;
-  t->split_cap = 0;
-  // [counts(32 words, one line)] [find indices n] [insert indices n] [update/erase indices n]
-  // [leader_of n] [combining table combine_slots(n)]
-  if (cudaMalloc(&t->split_idx, (32u + 4ull * n + combine_slots(n)) * sizeof(uint32_t)) != cudaSuccess)
-    return MT_ERR_OOM;
-  t->split_cap = n;
+  if (t->combine_mem) cudaFree(t->combine_mem);
+  t->combine_mem = nullptr;
+  t->combine_cap = 0;
+  if (cudaMalloc(&t->combine_mem, ((size_t)n + combine_slots(n)) * sizeof(uint32_t)) != cudaSuccess) return MT_ERR_OOM;
+  t->combine_cap = n;
   return MT_OK;
 }
 
-// Combine the updates among the requests `a` describes (a class of a mixed
-// batch, or a whole update call) on stream s; returns a.leader_of for the batch
-// kernel (nullptr when there is nothing to combine into).
-int launch_combine(mt_masstree* t, batch_args& a, uint32_t n, cudaStream_t s) {
-  uint32_t* leader_of = t->split_idx + 32 + 3ull * t->split_cap;
-  uint32_t* table = leader_of + t->split_cap;
-  const uint32_t slots = combine_slots(n);
-  if (cudaMemsetAsync(leader_of, 0xFF, (size_t)n * sizeof(uint32_t), s) != cudaSuccess ||
-      cudaMemsetAsync(table, 0xFF, (size_t)slots * sizeof(uint32_t), s) != cudaSuccess)
-    return MT_ERR_CUDA;
-  combine_kernel<<<std::max(1, std::min(t->sms * 8, (int)((n + 255) / 256))), 256, 0, s>>>(a, table, slots - 1u,
-                                                                                           leader_of);
+// Combine the updates among the requests of `a` on stream s and set
+// a.leader_of for the kernels that follow.
+int launch_combine(mt_masstree* t, batch_args& a, cudaStream_t s) {
+  int rc = ensure_combine_scratch(t, a.n, s);
+  if (rc) return rc;
+  const uint32_t slots = combine_slots(a.n);
+  uint32_t* table = t->combine_mem;
+  uint32_t* leader_of = table + slots;
+  if (cudaMemsetAsync(table, 0xFF, ((size_t)slots + a.n) * sizeof(uint32_t), s) != cudaSuccess) return MT_ERR_CUDA;
+  combine_kernel<<<std::max(1, std::min(t->sms * 8, (int)((a.n + 255) / 256))), 256, 0, s>>>(a, table, slots - 1u,
+                                                                                             leader_of);
   if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
   a.leader_of = leader_of;
   return MT_OK;
@@ -455,47 +451,14 @@ int launch_combine_results(mt_masstree* t, const batch_args& a, uint32_t n, cuda
   return cuda_status(cudaGetLastError());
 }
 
-int launch_mixed_split(mt_masstree* t, batch_args a, bool bucket_keys, cudaStream_t s) {
+// A mixed batch: the requests have no order among each other, so each lane
+// serves its own, whatever its kind (a walk is the same for all kinds).
+int launch_mixed(mt_masstree* t, batch_args a, cudaStream_t s) {
   if (a.n == 0) return MT_OK;
-  int rc = ensure_split_scratch(t, a.n, s);
-  if (rc) return rc;
-  rc = launch_reclaim(t, s);
-  if (rc) return rc;
-  uint32_t* counts = t->split_idx;
-  uint32_t* find_idx = t->split_idx + 32;
-  uint32_t* insert_idx = find_idx + a.n;
-  uint32_t* upderase_idx = insert_idx + a.n;
-  if (cudaMemsetAsync(counts, 0, 6 * sizeof(uint32_t), s) != cudaSuccess) return MT_ERR_CUDA;
-  partition3_kernel<<<std::max(1, std::min(t->sms * 8, (int)((a.n + 255) / 256))), 256, 0, s>>>(
-      a.types, a.key_lengths, a.max_key_length, bucket_keys ? 1u : 0u, a.n, find_idx, insert_idx, upderase_idx,
-      counts);
-  if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
-  batch_args f = a, i = a, u = a;
-  uint32_t* idx[3] = {find_idx, insert_idx, upderase_idx};
-  batch_args* cls[3] = {&f, &i, &u};
-  for (int c = 0; c < 3; ++c) {
-    cls[c]->index = idx[c];
-    cls[c]->n_dev = counts + 2 * c;
-    cls[c]->n_back_dev = counts + 2 * c + 1;
-    cls[c]->region = a.n;
-  }
-  // One launch per class, each compiled for its class only.
-  // The classes of one mixed batch have no order among each other, so they
-  // go to three streams (the caller's and two of the tree's, forked and
-  // joined by events): the blocks of one class fill the SMs that another
-  // class's tail leaves idle.
-  rc = host_fork(t, s);
-  if (rc) return rc;
-  // Write classes run with 16- or 32-lane tiles (narrower write tiles, allowed
-  // for plain insert/update/erase calls, are widened to 16 here).
-  const uint32_t tw = t->write_tile_size <= 16 ? 16u : 32u;
-  const uint32_t tu = t->upderase_tile_size ? t->upderase_tile_size : tw;
-  rc = launch_batch_tile<OP_PASS_INSERT, true>(t, tw, i, s);
-  if (!rc) rc = launch_find<true>(t, f, t->side[0]);
-  if (!rc) rc = launch_combine(t, u, a.n, t->side[1]);
-  if (!rc) rc = launch_batch_tile<OP_PASS_UPDERASE, true>(t, tu, u, t->side[1]);
-  if (!rc) rc = launch_combine_results(t, u, a.n, t->side[1]);
-  return host_join(t, s, rc);
+  int rc = launch_combine(t, a, s);
+  if (!rc) rc = launch_lane<OP_MIXED>(t, a, t->write_tile_size <= 16 ? 16u : 32u, s);
+  if (!rc) rc = launch_combine_results(t, a, a.n, s);
+  return rc;
 }
 
 template <int T, bool CONC>
@@ -552,7 +515,9 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
   const size_t stack_bytes = nslabs * 4u;
   const size_t ctr_bytes = (size_t)kShards * 3u * kCtrStride * sizeof(int);
   const size_t err_bytes = 128;
-  const size_t total = slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes;
+  // The defer list of the lane kernels: 1/256 of the pool, at most 1M entries.
+  const uint64_t defer_cap = std::min<uint64_t>(1u << 20, std::max<uint64_t>(4096u, pool_bytes / 1024u));
+  const size_t total = slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes + 128 + defer_cap * 4u;
   if (cudaMalloc(&t->mem, total) != cudaSuccess) { delete t; return MT_ERR_OOM; }
   char* base = (char*)t->mem;
   pool_view& p = t->tv.pool;
@@ -561,6 +526,8 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
   p.limbo = (uint32_t*)(base + slab_bytes + stack_bytes);
   p.ctr = (int*)(base + slab_bytes + 2 * stack_bytes);
   p.err = (uint32_t*)(base + slab_bytes + 2 * stack_bytes + ctr_bytes);
+  t->defer_mem = (uint32_t*)(base + slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes);
+  t->defer_cap = (uint32_t)defer_cap;
   p.num_slabs = (uint32_t)nslabs;
   p.num_shards = kShards;
   p.shard_slabs = shard_slabs;
@@ -591,7 +558,7 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
 
 namespace mtb {
 int host_launch_insert(mt_masstree* t, const batch_args& a, bool upsert, cudaStream_t s) {
-  return upsert ? launch_batch<OP_UPSERT, true>(t, a, s) : launch_batch<OP_INSERT, true>(t, a, s);
+  return upsert ? launch_lane<OP_UPSERT>(t, a, s) : launch_lane<OP_INSERT>(t, a, s);
 }
 }  // namespace mtb
 
@@ -626,7 +593,7 @@ int mt_destroy(mt_masstree* t) {
   if (!t) return MT_ERR_INVALID_ARG;
   cudaDeviceSynchronize();
   if (t->frames) cudaFree(t->frames);
-  if (t->split_idx) cudaFree(t->split_idx);
+  if (t->combine_mem) cudaFree(t->combine_mem);
   if (t->batches_mem) cudaFree(t->batches_mem);
   if (t->grouped_mem) cudaFree(t->grouped_mem);
   if (t->merge_log) cudaFree(t->merge_log);
@@ -720,7 +687,7 @@ int mt_insert(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_
     }
   }
   if (n) t->maybe_empty = false;
-  return upsert ? launch_batch<OP_UPSERT, true>(t, a, s) : launch_batch<OP_INSERT, true>(t, a, s);
+  return upsert ? launch_lane<OP_UPSERT>(t, a, s) : launch_lane<OP_INSERT>(t, a, s);
 }
 
 int mt_update(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_t* klens, const uint32_t* values,
@@ -731,10 +698,9 @@ int mt_update(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_
   a.keys = keys; a.key_lengths = klens; a.values = const_cast<uint32_t*>(values); a.value_lengths_in = vlens;
   a.results = results; a.max_key_length = maxK; a.max_value_length = maxV; a.n = n;
   const cudaStream_t s = (cudaStream_t)stream;
-  if (n < 2) return launch_batch<OP_UPDATE, true>(t, a, s);
-  int rc = ensure_split_scratch(t, n, s);
-  if (!rc) rc = launch_combine(t, a, n, s);
-  if (!rc) rc = launch_batch<OP_UPDATE, true>(t, a, s);
+  if (n < 2) return launch_lane<OP_UPDATE>(t, a, s);
+  int rc = launch_combine(t, a, s);
+  if (!rc) rc = launch_lane<OP_UPDATE>(t, a, s);
   if (!rc) rc = launch_combine_results(t, a, n, s);
   return rc;
 }
@@ -745,10 +711,10 @@ int mt_erase(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_t
   batch_args a{};
   a.keys = keys; a.key_lengths = klens; a.results = results; a.max_key_length = maxK; a.n = n;
   const cudaStream_t s = (cudaStream_t)stream;
-  if (!(flags & (MT_FLAG_MERGE | MT_FLAG_REMOVE_EMPTY_LAYERS))) return launch_batch<OP_ERASE, true>(t, a, s);
+  if (!(flags & (MT_FLAG_MERGE | MT_FLAG_REMOVE_EMPTY_LAYERS))) return launch_lane<OP_ERASE>(t, a, s);
   const int rc = host_merge_begin(t, s, flags);
   if (rc) return rc;
-  return host_merge_end(t, s, launch_batch<OP_ERASE, true>(t, a, s));
+  return host_merge_end(t, s, launch_lane<OP_ERASE>(t, a, s));
 }
 
 int mt_mixed_batch(mt_masstree* t, const uint8_t* types, const uint32_t* keys, uint32_t maxK,
@@ -761,8 +727,8 @@ int mt_mixed_batch(mt_masstree* t, const uint8_t* types, const uint32_t* keys, u
   a.max_key_length = maxK; a.max_value_length = maxV; a.n = n;
   const cudaStream_t s = (cudaStream_t)stream;
   auto run = [&] {
-    if (flags & MT_FLAG_SINGLE_PASS) return launch_batch<OP_MIXED, true>(t, a, s);
-    return launch_mixed_split(t, a, (flags & MT_FLAG_BUCKET_KEYS) != 0, s);
+    if (flags & MT_FLAG_SINGLE_PASS) return launch_single_pass(t, a, s);
+    return launch_mixed(t, a, s);
   };
   if (!(flags & (MT_FLAG_MERGE | MT_FLAG_REMOVE_EMPTY_LAYERS))) return run();
   const int rc = host_merge_begin(t, s, flags);

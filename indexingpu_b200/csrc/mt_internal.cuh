@@ -22,6 +22,9 @@ constexpr uint32_t kClassBarrierMin = 1u << 17;
 #ifndef MT_LANE_FIND_BLOCKS
 #define MT_LANE_FIND_BLOCKS 6  // occupancy hint for the find kernels (one request per thread)
 #endif
+#ifndef MT_LANE_WRITE_BLOCKS
+#define MT_LANE_WRITE_BLOCKS 4  // and for the write and mixed kernels (an image, an edit and a fence: 128 registers)
+#endif
 #ifndef MT_WRITE_MIN_BLOCKS_PER_SM
 #define MT_WRITE_MIN_BLOCKS_PER_SM MT_MIN_BLOCKS_PER_SM  // the same for kernels that insert
 #endif
@@ -59,6 +62,7 @@ struct batch_args {
   uint32_t max_key_length;
   uint32_t max_value_length;
   uint32_t n;
+  uint32_t first;              // lane kernels: serve requests (or index entries) first .. first + n
 };
 
 struct scan_args {
@@ -217,8 +221,10 @@ struct mt_masstree {
   uint32_t upderase_tile_size = 0;  // updates and erases of mixed batches (0: the write width)
   uint32_t scan_tile_size = 0;   // scans (0: the find width)
   uint32_t blocks_per_sm = 0;    // 0 = occupancy limit
-  uint32_t* split_idx = nullptr; // mixed-batch partition scratch
-  uint32_t split_cap = 0;
+  uint32_t* combine_mem = nullptr;  // update-combining scratch (grown on demand)
+  uint32_t combine_cap = 0;
+  uint32_t* defer_mem = nullptr;    // requests the lane kernels hand on: count (one line), then defer_cap entries
+  uint32_t defer_cap = 0;
   // Streams and events of the forked class launches of large mixed batches
   // (created on first use).
   cudaStream_t side[2] = {nullptr, nullptr};

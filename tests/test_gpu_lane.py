@@ -55,3 +55,73 @@ def test_finds_at_slab_edges(n, maxK, maxV):
                     np.testing.assert_array_equal(gv, ov)
     finally:
         g.close()
+
+
+def _same_contents(g, o, n, maxK, maxV):
+    lower, one = np.zeros((1, maxK), np.uint32), np.ones(1, np.uint32)
+    for x, y, what in zip(g.scan(lower, one, n + 2, maxV=maxV), o.scan(lower, one, n + 2, maxV=maxV),
+                          ("counts", "values", "value lengths", "keys", "key lengths")):
+        np.testing.assert_array_equal(x, y, err_msg=what)
+    ok, keys, msg = g.t.validate()
+    assert ok and keys == len(o.dump(maxK, maxV)[1]), msg
+
+
+@pytest.mark.parametrize("n", [1, 33, 4000, 120000])
+@pytest.mark.parametrize("maxK,maxV", [(1, 1), (9, 8), (32, 30), (63, 62)])
+def test_mixed_batches_at_slab_edges(n, maxK, maxV):
+    # Touch-once batches of every kind: each request's result is defined.
+    keys, kl, vals, vl = _edge_keys(n, maxK, maxV, 11 * n + maxV)
+    m = len(kl)
+    rng = np.random.default_rng(n)
+    g, o = GpuIndex(pool_bytes=512 << 20), OracleIndex()
+    try:
+        held = rng.permutation(m)[:m // 2]
+        if len(held):
+            np.testing.assert_array_equal(g.insert(keys[held], kl[held], vals[held], vl[held]),
+                                          o.insert(keys[held], kl[held], vals[held], vl[held]))
+        for _ in range(3):
+            types = rng.integers(0, 4, m).astype(np.uint8)
+            v = rng.integers(1, 1 << 32, (m, maxV), dtype=np.uint64).astype(np.uint32)
+            l = rng.permutation(vl)
+            order = rng.permutation(m)
+            gv, gl, gr = g.mixed(types, keys[order], kl[order], v, l)
+            ov, ol, orr = o.mixed(types, keys[order], kl[order], v, l)
+            find = types == 2
+            np.testing.assert_array_equal(gr[~find], orr[~find])
+            np.testing.assert_array_equal(gl[find], ol[find])
+            live = np.arange(maxV)[None, :] < np.minimum(ol, maxV)[:, None]
+            assert (np.where(live, gv, 0)[find] == np.where(live, ov, 0)[find]).all()
+        _same_contents(g, o, m, maxK, maxV)
+    finally:
+        g.close()
+
+
+@pytest.mark.parametrize("upsert", [False, True])
+def test_writes_that_meet_in_one_node(upsert):
+    # Ascending keys inserted beside each other split the same nodes again and
+    # again; many requests then write and erase few keys.
+    n = 30000
+    g, o = GpuIndex(pool_bytes=256 << 20), OracleIndex()
+    try:
+        keys = np.arange(3 * n, dtype=np.uint32)[:, None]
+        one = np.ones(n, np.uint32)
+        for i in range(3):  # the first call builds, the others insert between and after
+            k = keys[i::3] if i < 2 else keys[2::3] + np.uint32(5 * n)
+            np.testing.assert_array_equal(g.insert(k, one, k + 1, one, upsert=upsert),
+                                          o.insert(k, one, k + 1, one, upsert=upsert))
+        _same_contents(g, o, 3 * n, 1, 1)
+        few = np.repeat(keys[:60][np.arange(60) % 3 != 2], 200, axis=0)  # 40 keys
+        ones = np.ones(len(few), np.uint32)
+        assert g.update(few, ones, few + 7, ones).all()
+        o.update(few, ones, few + 7, ones)
+        _same_contents(g, o, 3 * n, 1, 1)
+        erased = g.erase(few, ones)
+        o.erase(few, ones)
+        assert int(erased.sum()) == 40 and (np.bincount(few[:, 0], erased)[np.unique(few)] == 1).all()
+        _same_contents(g, o, 3 * n, 1, 1)
+        added = g.insert(few, ones, few + 9, ones, upsert=upsert)
+        o.insert(few, ones, few + 9, ones, upsert=upsert)
+        assert int(added.sum()) == (len(few) if upsert else 40)
+        _same_contents(g, o, 3 * n, 1, 1)
+    finally:
+        g.close()
