@@ -539,7 +539,7 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
   root_img[WORD_SIB] = kInvalid;
   root_img[WORD_META] = META_BORDER | META_ROOT;
   root_img[WORD_KS] = 0u;
-  root_img[WORD_CSUM] = node_checksum(root_img);
+  seal_image(root_img);
   const int one = 1;
   if (e == cudaSuccess) e = cudaMemcpy(p.slabs, root_img, sizeof(root_img), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(p.bump(0), &one, sizeof(int), cudaMemcpyHostToDevice);
@@ -903,7 +903,7 @@ struct validator {
     }
     last[level] = idx;
     if (n > (uint32_t)kMaxEntries) return fail("count above the node capacity");
-    if (node_checksum(w) != w[WORD_CSUM]) return fail("node checksum mismatch");
+    if (node_checksum(w) != stored_checksum(w)) return fail("node checksum mismatch");
     if (w[WORD_HIGH] != hi) return fail("high key differs from the parent's separator");
     const bool border = (meta & META_BORDER) != 0;
     if (border) {

@@ -35,46 +35,59 @@ MT_DEV void lane_load_relaxed(const uint32_t* a, uint32_t (&w)[32]) {
                  : "l"(a + 8 * q) : "memory");
 }
 
-MT_DEV uint32_t lane_checksum(const uint32_t (&w)[32]) {
-  uint32_t h = 0;
+// Out of line: errors are rare, and inlined recording would crowd the
+// instruction cache.
+static __device__ __noinline__ void lane_error(uint32_t* err, uint32_t code, uint32_t site) {
+  pool_view p{};
+  p.err = err;
+  record_error(p, code, site);
+}
+
+MT_DEV uint64_t lane_checksum(const uint32_t (&w)[32]) {
+  uint64_t h = kCsumInit;
 #pragma unroll
   for (int g = 0; g < 32; ++g) h += csum_term((uint32_t)g, w[g]);
   return h;
 }
-
-// A verified image of node i (bounded reloads, as node::load_verified).
-template <bool CONC>
-MT_DEV bool lane_read_node(const pool_view& p, uint32_t i, uint32_t (&w)[32]) {
-  lane_load_weak(p.addr(i), w);
-  if (!CONC) return true;
-  for (uint32_t r = 0; lane_checksum(w) != w[WORD_CSUM]; ++r) {
-    if (r >= kTornRetries) {
-      record_error(p, ERR_CORRUPT, MT_AT(SRC_LANE));
-      return false;
-    }
-    lane_load_relaxed(p.addr(i), w);
-  }
-  return true;
+MT_DEV bool lane_verify(const uint32_t (&w)[32]) {
+  return lane_checksum(w) == ((uint64_t)w[WORD_CSUM + 1] << 32 | w[WORD_CSUM]);
+}
+MT_DEV void lane_seal(uint32_t (&w)[32]) {
+  const uint64_t h = lane_checksum(w);
+  w[WORD_CSUM] = (uint32_t)h;
+  w[WORD_CSUM + 1] = (uint32_t)(h >> 32);
 }
 
-// The same from L2: the node's latest published image.
-MT_DEV bool lane_read_fresh(const pool_view& p, uint32_t i, uint32_t (&w)[32]) {
-  lane_load_relaxed(p.addr(i), w);
-  for (uint32_t r = 0; lane_checksum(w) != w[WORD_CSUM]; ++r) {
-    if (r >= kTornRetries) {
-      record_error(p, ERR_CORRUPT, MT_AT(SRC_LANE));
-      return false;
-    }
-    lane_load_relaxed(p.addr(i), w);
+// First entry at or after (slice, more) in an image's order: its position (the
+// count if there is none), and its words.  An interior node's separators count
+// as continuing keys, so the first one >= slice is found, whose child covers it.
+// (Entry words past the count are 0 and never precede a found entry.)
+MT_DEV uint32_t lane_search(const uint32_t (&w)[32], uint32_t slice, bool more, uint32_t& key, uint32_t& val) {
+  uint32_t pos = kMaxEntries;
+  key = val = 0u;
+#pragma unroll
+  for (int e = kMaxEntries - 1; e >= 0; --e) {
+    const bool c = w[2 * e] >= slice;
+    pos = c ? (uint32_t)e : pos;
+    key = c ? w[2 * e] : key;
+    val = c ? w[2 * e + 1] : val;
   }
-  return true;
+  if (more && key == slice && (w[WORD_META] & META_BORDER) && pos < (w[WORD_META] & META_COUNT) &&
+      !(ks_get(w[WORD_KS], pos) & KS_MORE)) {
+    // The key that ends at this slice comes first: the next entry.
+    ++pos;
+    key = val = 0u;
+#pragma unroll
+    for (int e = 1; e < kMaxEntries; ++e) {
+      key = (uint32_t)e == pos ? w[2 * e] : key;
+      val = (uint32_t)e == pos ? w[2 * e + 1] : val;
+    }
+  }
+  return min(pos, w[WORD_META] & META_COUNT);
 }
-
-// Bits 2e of the entries e < n of a border node whose key continues past its
-// slice (more) or ends at it (!more).
-MT_DEV uint32_t lane_eligible(uint32_t meta, uint32_t ks, bool more) {
-  const uint32_t n = meta & META_COUNT;
-  return (more ? ks : ~ks) & 0x01555555u & ((1u << (2u * n)) - 1u);
+// Whether the entry a search ended at is the one for (slice, more).
+MT_DEV bool lane_is_entry(uint32_t meta, uint32_t ks, uint32_t pos, uint32_t key, uint32_t slice, bool more) {
+  return pos < (meta & META_COUNT) && key == slice && ((ks_get(ks, pos) & KS_MORE) != 0u) == more;
 }
 
 // Where a request's key belongs: the border node of its last layer and, when
@@ -87,67 +100,75 @@ struct lane_place {
   uint32_t state;   // the entry's key state
   uint32_t val;     // the entry's value word
   bool found;
+  bool full;        // the border node has no room (and is not a layer root)
 };
 
-// Walk from the root of layer 0 to the key's place.  False on a (recorded)
-// error.
+// Walk from the root of layer 0 to the key's place, for the lanes with `go`
+// (klen > 0); called by the whole warp.  The warp goes round the loop together,
+// one node visit per lane and round: left to themselves, lanes in interior and
+// border nodes drift apart and run the loop one after the other.  go is
+// cleared after a (recorded) error.
 template <bool CONC>
-MT_DEV bool lane_locate(const tree_view& tv, const uint32_t* key, uint32_t klen, lane_place& at) {
+MT_DEV void lane_locate(const tree_view& tv, bool& go, const uint32_t* key, uint32_t klen, lane_place& at) {
   const pool_view& p = tv.pool;
-  uint32_t idx = tv.root, layer = 0, hops = 0;
-  uint32_t slice = key[0];
+  uint32_t idx = tv.root, hops = 0, torn = 0;
+  uint32_t slice = go ? key[0] : 0u;
   bool more = klen > 1u;
-  uint32_t w[32];
+  bool walk = go;
   at.found = false;
   at.layer = 0;
   at.parent = kInvalid;
   at.root = idx;
-  while (true) {
-    if (!p.valid(idx) || ++hops > kMaxHops) {
-      record_error(p, ERR_CORRUPT, MT_AT(SRC_LANE));
-      return false;
-    }
-    if (!lane_read_node<CONC>(p, idx, w)) return false;
-    const uint32_t meta = w[WORD_META];
-    if ((meta & META_SIB) && slice > w[WORD_HIGH]) {
-      idx = w[WORD_SIB];
-      continue;
-    }
-    if (!(meta & META_BORDER)) {
-      // The first separator >= slice; separators past the count are skipped.
-      const uint32_t n = meta & META_COUNT;
-      uint32_t child = kInvalid;
-#pragma unroll
-      for (int e = kMaxEntries - 1; e >= 0; --e)
-        if ((uint32_t)e < n && slice <= w[2 * e]) child = w[2 * e + 1];
-      at.parent = idx;
-      idx = child;  // none: caught as an invalid slab above
-      continue;
-    }
-    const uint32_t ok = lane_eligible(meta, w[WORD_KS], more);
-    uint32_t hit = 0, val = 0;
-#pragma unroll
-    for (int e = 0; e < kMaxEntries; ++e)
-      if (w[2 * e] == slice && (ok & (1u << (2 * e)))) {
-        hit = 1u << (2 * e);
-        val = w[2 * e + 1];
+#pragma unroll 1
+  while (__any_sync(0xFFFFFFFFu, walk)) {
+    if (walk) {
+      uint32_t err = ERR_NONE;
+      if (!p.valid(idx) || ++hops > kMaxHops) {
+        err = ERR_CORRUPT;
+      } else {
+        uint32_t w[32];
+        if (CONC && torn != 0u) lane_load_relaxed(p.addr(idx), w);
+        else lane_load_weak(p.addr(idx), w);
+        if (CONC && !lane_verify(w)) {  // read again, from L2 (bounded, as node::load_verified)
+          --hops;
+          if (++torn > kTornRetries) err = ERR_CORRUPT;
+        } else {
+          torn = 0;
+          const uint32_t meta = w[WORD_META];
+          const bool border = (meta & META_BORDER) != 0u;
+          uint32_t k, v;
+          const uint32_t pos = lane_search(w, slice, more, k, v);
+          if ((meta & META_SIB) && slice > w[WORD_HIGH]) {
+            idx = w[WORD_SIB];
+          } else if (!border) {
+            at.parent = idx;
+            idx = pos < (meta & META_COUNT) ? v : kInvalid;  // none: caught as an invalid slab above
+          } else {
+            const uint32_t state = ks_get(w[WORD_KS], pos);
+            const bool hit = lane_is_entry(meta, w[WORD_KS], pos, k, slice, more);
+            if (hit && state == KS_LINK) {
+              idx = v;
+              at.root = v;
+              at.parent = kInvalid;
+              ++at.layer;
+              slice = key[at.layer];
+              more = at.layer + 1u < klen;
+            } else {
+              at.idx = idx;
+              at.full = (meta & (META_COUNT | META_ROOT)) == (uint32_t)kMaxEntries;
+              at.found = hit;
+              at.state = state;
+              at.val = v;
+              walk = false;
+            }
+          }
+        }
       }
-    at.layer = layer;
-    at.idx = idx;
-    if (!hit) return true;
-    const uint32_t state = (more ? KS_MORE : 0u) | ((w[WORD_KS] & (hit << 1)) ? KS_SLAB : 0u);
-    if (state != KS_LINK) {
-      at.found = true;
-      at.state = state;
-      at.val = val;
-      return true;
+      if (err != ERR_NONE) {
+        lane_error(p.err, err, MT_AT(SRC_LANE));
+        walk = go = false;
+      }
     }
-    idx = val;
-    at.root = val;
-    at.parent = kInvalid;
-    ++layer;
-    slice = key[layer];
-    more = layer + 1u < klen;
   }
 }
 
@@ -156,18 +177,20 @@ MT_DEV bool lane_locate(const tree_view& tv, const uint32_t* key, uint32_t klen,
 // and out is not null, copy at most maxV value slices.  Eight lanes serve one
 // request, lane r of them the words r, r+8, r+16 and r+24 of a slab: every load
 // and store covers whole 32-byte sectors of four requests' lines.  Only the
-// sectors that the key rest and maxV value slices can reach are read, and four
+// sectors that the key rest and maxV value slices can reach are read, and two
 // requests' loads (per eight lanes) are in flight together.  Called by the
-// whole warp; eq and vlen are set for the lanes with want.
+// whole warp; eq and vlen are set for the lanes with want.  (Every vote and
+// shuffle stands alone: none may be skipped by a lane's && or ?:.)
 template <bool VALUES>
 MT_DEV void warp_chains(const pool_view& p, bool want, uint32_t head, const uint32_t* K, uint32_t lk, uint32_t* out,
                         uint32_t maxV, bool& eq, uint32_t& vlen) {
-  constexpr int kRound = 4;
+  constexpr int kRound = MT_CHAIN_ROUND;
   const uint32_t lane = lane_id();
   const uint32_t r8 = lane & 7u, first = lane & 24u;
   const uint32_t todo = __ballot_sync(0xFFFFFFFFu, want);
   if (todo == 0u) return;
   const uint32_t columns = todo | (todo >> 8) | (todo >> 16) | (todo >> 24);  // bit i: lane i of some eight lanes
+#pragma unroll 1
   for (int base = 0; base < 8; base += kRound) {
     if (!((columns >> base) & ((1u << kRound) - 1u))) continue;
     uint32_t c[kRound][4], kw[kRound][4];
@@ -175,8 +198,8 @@ MT_DEV void warp_chains(const pool_view& p, bool want, uint32_t head, const uint
     for (int i = 0; i < kRound; ++i) {
       const uint32_t src = first + base + i;
       const uint32_t hd = __shfl_sync(0xFFFFFFFFu, head, src);
-      const uint32_t need = __shfl_sync(0xFFFFFFFFu, lk, src) + (VALUES ? maxV : 0u);
-      const uint32_t n = min(__shfl_sync(0xFFFFFFFFu, lk, src), kSufData);
+      const uint32_t n = __shfl_sync(0xFFFFFFFFu, lk, src);
+      const uint32_t need = n + (VALUES ? maxV : 0u);
       const uint32_t* k = reinterpret_cast<const uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(K), src));
       const bool act = (todo >> src) & 1u;
       const uint32_t* a = p.addr(act ? hd : 0u) + r8;
@@ -185,7 +208,7 @@ MT_DEV void warp_chains(const pool_view& p, bool want, uint32_t head, const uint
         const uint32_t g = r8 + 8u * q;
         c[i][q] = 0u;
         if (act && (g < need || g >= kSufData)) c[i][q] = a[8 * q];
-        kw[i][q] = (act && g < n) ? k[g] : 0u;
+        kw[i][q] = (act && g < n && g < kSufData) ? k[g] : 0u;
       }
     }
 #pragma unroll
@@ -193,60 +216,70 @@ MT_DEV void warp_chains(const pool_view& p, bool want, uint32_t head, const uint
       const uint32_t src = first + base + i;
       const bool act = (todo >> src) & 1u;
       const uint32_t n = __shfl_sync(0xFFFFFFFFu, lk, src);
-      const uint32_t* k = reinterpret_cast<const uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(K), src));
       const uint32_t hdr = __shfl_sync(0xFFFFFFFFu, c[i][3], first + SUF_WORD_HDR % 8);
-      uint32_t nx = __shfl_sync(0xFFFFFFFFu, c[i][3], first + SUF_WORD_NEXT % 8);
-      const uint32_t vl = hdr >> 16;
-      bool same = (hdr & kMaxLen16) == n;
+      bool differs = act && (hdr & kMaxLen16) != n;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t g = r8 + 8u * q;
+        differs |= act && g < kSufData && g < n && c[i][q] != kw[i][q];
+      }
+      const uint32_t other = __ballot_sync(0xFFFFFFFFu, differs);
+      const bool same = !((other >> first) & 0xFFu);
+      if (VALUES) {
+        uint32_t* o = reinterpret_cast<uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(out), src));
+        const uint32_t last = n + min(hdr >> 16, maxV);  // data slices [0, n) are compared, [n, last) copied
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t g = r8 + 8u * q;
+          if (act && same && o != nullptr && g < kSufData && g >= n && g < last) o[g - n] = c[i][q];
+        }
+      }
+      if (r8 == (uint32_t)(base + i)) {
+        eq = same;
+        vlen = hdr >> 16;
+      }
+    }
+  }
+  // Chains of several slabs: the slabs after the head, one request per eight
+  // lanes at a time.
+  uint32_t last = want && eq ? lk + (VALUES && out != nullptr ? min(vlen, maxV) : 0u) : 0u;
+  const uint32_t longer = __ballot_sync(0xFFFFFFFFu, last > kSufData);
+  if (longer == 0u) return;
+#pragma unroll 1
+  for (uint32_t i = 0; i < 8u; ++i) {
+    const uint32_t src = first + i;
+    const uint32_t n = __shfl_sync(0xFFFFFFFFu, lk, src);
+    const uint32_t hd = __shfl_sync(0xFFFFFFFFu, head, src);
+    const uint32_t* k = reinterpret_cast<const uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(K), src));
+    uint32_t* o = reinterpret_cast<uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(out), src));
+    const uint32_t end = __shfl_sync(0xFFFFFFFFu, last, src);
+    bool same = end > kSufData;
+    uint32_t nx = same ? p.addr(hd)[SUF_WORD_NEXT] : kInvalid;
+#pragma unroll 1
+    for (uint32_t at = kSufData; __any_sync(0xFFFFFFFFu, same && at < end); at += kSufData) {
+      const bool on = same && at < end && p.valid(nx);
+      if (same && !on && at < n) same = false;  // a chain cut short cannot hold the key
+      uint32_t d[4];
       bool differs = false;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const uint32_t g = r8 + 8u * q;
-        if (act && g < kSufData && g < n) differs |= c[i][q] != kw[i][q];
+        d[q] = on ? p.addr(nx)[g] : 0u;
+        if (on && g < kSufData && at + g < n) differs |= d[q] != k[at + g];
       }
-      const uint32_t other = __ballot_sync(0xFFFFFFFFu, differs);  // by every lane, whatever `same` is
-      same = same && !((other >> first) & 0xFFu);
-      uint32_t* o = nullptr;
-      uint32_t last = n;  // data slices [0, n) are compared, [n, last) copied
+      const uint32_t rest = __ballot_sync(0xFFFFFFFFu, differs);
+      if ((rest >> first) & 0xFFu) same = false;
       if (VALUES) {
-        o = reinterpret_cast<uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(out), src));
-        if (o != nullptr) last = n + min(vl, maxV);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const uint32_t g = r8 + 8u * q;
-          if (act && same && g < kSufData && g >= n && g < last) o[g - n] = c[i][q];
+          if (on && same && g < kSufData && at + g >= n && at + g < end) o[at + g - n] = d[q];
         }
       }
-      // Chains of several slabs.
-      for (uint32_t at = kSufData; __any_sync(0xFFFFFFFFu, act && same && at < last); at += kSufData) {
-        const bool on = act && same && at < last && p.valid(nx);
-        same = same && (on || at >= last || at >= n);  // a chain cut short cannot hold the key
-        uint32_t d[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) d[q] = on ? p.addr(nx)[r8 + 8u * q] : 0u;
-        differs = false;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t g = r8 + 8u * q;
-          if (on && g < kSufData && at + g < n) differs |= d[q] != k[at + g];
-        }
-        const uint32_t rest = __ballot_sync(0xFFFFFFFFu, differs);
-        same = same && !((rest >> first) & 0xFFu);
-        if (VALUES) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint32_t g = r8 + 8u * q;
-            if (on && same && g < kSufData && at + g >= n && at + g < last) o[at + g - n] = d[q];
-          }
-        }
-        nx = __shfl_sync(0xFFFFFFFFu, d[3], first + SUF_WORD_NEXT % 8);
-        if (!on) nx = kInvalid;
-      }
-      if ((lane & 7u) == (uint32_t)(base + i)) {
-        eq = same;
-        vlen = vl;
-      }
+      nx = __shfl_sync(0xFFFFFFFFu, d[3], first + SUF_WORD_NEXT % 8);
+      if (!on) nx = kInvalid;
     }
+    if (r8 == i && last > kSufData) eq = same;
   }
 }
 
@@ -272,6 +305,7 @@ MT_DEV void lane_find(const tree_view& tv, const batch_args& a) {
   const uint32_t n = nf + nb;
   const uint32_t per = max(1u, min(32u, (n + warps - 1u) / warps));
   uint32_t* values = a.values_out ? a.values_out : a.values;
+#pragma unroll 1
   for (uint32_t base = warp * per; base < n; base += warps * per) {
     if (__any_sync(0xFFFFFFFFu, slot == 0u && fatal_error(p))) break;
     const uint32_t pos = base + slot;
@@ -282,17 +316,17 @@ MT_DEV void lane_find(const tree_view& tv, const batch_args& a) {
       klen = a.key_lengths ? a.key_lengths[i] : a.max_key_length;
     }
     const bool bad = valid && klen > a.max_key_length;
-    if (bad) record_error(p, ERR_INVALID_ARG);
+    if (bad) lane_error(p.err, ERR_INVALID_ARG, MT_AT(SRC_LANE));
     const uint32_t* key = a.keys + (size_t)i * a.max_key_length;
     uint32_t* out = values ? values + (size_t)i * a.max_value_length : nullptr;
     lane_place at;
-    at.found = false;
-    at.layer = 0;
-    if (valid && !bad && klen > 0u && !lane_locate<CONC>(tv, key, klen, at)) at.found = false;
+    bool go = valid && !bad && klen > 0u;
+    lane_locate<CONC>(tv, go, key, klen, at);
+    if (!go) at.found = false;
     uint32_t vlen = 0;
     bool chain = at.found && at.state != KS_VALUE;
     if (chain && !p.valid(at.val)) {
-      record_error(p, ERR_CORRUPT, MT_AT(SRC_LANE));
+      lane_error(p.err, ERR_CORRUPT, MT_AT(SRC_LANE));
       chain = false;
     }
     if (at.found && at.state == KS_VALUE) {
@@ -356,6 +390,7 @@ MT_DEV uint32_t lane_slab(const pool_view& p, const lane_slabs& s, uint32_t q) {
 MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, uint32_t& shard, lane_slabs& s) {
   const uint32_t lane = lane_id();
   bool got = need == 0u;
+#pragma unroll 1
   for (uint32_t k = 0; k < p.num_shards; ++k) {
     const uint32_t want = got ? 0u : need;
     uint32_t incl = want;
@@ -404,6 +439,7 @@ MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, uint32_t& shard, 
         got = true;
       } else {
         // The part of a lane's need that this shard covered goes back.
+#pragma unroll 1
         for (uint32_t q = g.first; q < have; ++q) retire_slab(p, lane_slab(p, g, q - g.first));
       }
     }
@@ -418,7 +454,7 @@ MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, uint32_t& shard, 
 // in warp_chains; whole 32-byte sectors are stored.
 MT_DEV void warp_write_chains(const pool_view& p, bool want, const lane_slabs& s, const uint32_t* K, uint32_t lk,
                               const uint32_t* V, uint32_t vlen, uint32_t& head) {
-  constexpr int kRound = 4;
+  constexpr int kRound = MT_CHAIN_ROUND;
   const uint32_t lane = lane_id();
   const uint32_t r8 = lane & 7u, first = lane & 24u;
   const uint32_t todo = __ballot_sync(0xFFFFFFFFu, want);
@@ -430,6 +466,7 @@ MT_DEV void warp_write_chains(const pool_view& p, bool want, const lane_slabs& s
     if (total > kSufData) next = lane_slab(p, s, 1u);
   }
   const uint32_t columns = todo | (todo >> 8) | (todo >> 16) | (todo >> 24);
+#pragma unroll 1
   for (int base = 0; base < 8; base += kRound) {
     if (!((columns >> base) & ((1u << kRound) - 1u))) continue;
     uint32_t c[kRound][4];
@@ -440,12 +477,11 @@ MT_DEV void warp_write_chains(const pool_view& p, bool want, const lane_slabs& s
       const uint32_t all = __shfl_sync(0xFFFFFFFFu, total, src);
       const uint32_t* k = reinterpret_cast<const uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(K), src));
       const uint32_t* v = reinterpret_cast<const uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(V), src));
-      const bool act = (todo >> src) & 1u;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const uint32_t g = r8 + 8u * q;
+        const uint32_t g = r8 + 8u * q;  // all: 0 for a request without a chain
         c[i][q] = 0u;
-        if (act && g < kSufData && g < all) c[i][q] = g < n ? k[g] : v[g - n];
+        if (g < kSufData && g < all) c[i][q] = *(g < n ? k + g : v + (g - n));
       }
     }
 #pragma unroll
@@ -462,31 +498,37 @@ MT_DEV void warp_write_chains(const pool_view& p, bool want, const lane_slabs& s
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         if (act) a[8 * q] = c[i][q];
-      if (!__any_sync(0xFFFFFFFFu, act && all > kSufData)) continue;
-      // Further slabs.
-      const uint32_t* k = reinterpret_cast<const uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(K), src));
-      const uint32_t* v = reinterpret_cast<const uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(V), src));
-      lane_slabs o;
-      o.shard = __shfl_sync(0xFFFFFFFFu, s.shard, src);
-      o.lo = __shfl_sync(0xFFFFFFFFu, s.lo, src);
-      o.n_stack = __shfl_sync(0xFFFFFFFFu, s.n_stack, src);
-      o.bump = __shfl_sync(0xFFFFFFFFu, s.bump, src);
-      o.first = __shfl_sync(0xFFFFFFFFu, s.first, src);
-      uint32_t cur = nx;
-      for (uint32_t at = kSufData, sl = 2u; act && at < all; at += kSufData, ++sl) {
-        const uint32_t after = at + kSufData < all ? lane_slab(p, o, sl) : kInvalid;
-        uint32_t* b = p.addr(cur) + r8;
+    }
+  }
+  // Further slabs, one request per eight lanes at a time.
+  if (!__any_sync(0xFFFFFFFFu, total > kSufData)) return;
+#pragma unroll 1
+  for (uint32_t i = 0; i < 8u; ++i) {
+    const uint32_t src = first + i;
+    const uint32_t n = __shfl_sync(0xFFFFFFFFu, lk, src);
+    const uint32_t all = __shfl_sync(0xFFFFFFFFu, total, src);
+    const uint32_t* k = reinterpret_cast<const uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(K), src));
+    const uint32_t* v = reinterpret_cast<const uint32_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(V), src));
+    uint32_t cur = __shfl_sync(0xFFFFFFFFu, next, src);
+    lane_slabs o;
+    o.shard = __shfl_sync(0xFFFFFFFFu, s.shard, src);
+    o.lo = __shfl_sync(0xFFFFFFFFu, s.lo, src);
+    o.n_stack = __shfl_sync(0xFFFFFFFFu, s.n_stack, src);
+    o.bump = __shfl_sync(0xFFFFFFFFu, s.bump, src);
+    o.first = __shfl_sync(0xFFFFFFFFu, s.first, src);
+#pragma unroll 1
+    for (uint32_t at = kSufData, sl = 2u; at < all; at += kSufData, ++sl) {
+      const uint32_t after = at + kSufData < all ? lane_slab(p, o, sl) : kInvalid;
+      uint32_t* b = p.addr(cur) + r8;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t g = r8 + 8u * q, di = at + g;
-          uint32_t x = 0u;
-          if (g < kSufData && di < all) x = di < n ? k[di] : v[di - n];
-          if (g == (uint32_t)SUF_WORD_NEXT) x = after;
-          b[8 * q] = x;
-        }
-        cur = after;
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t g = r8 + 8u * q, di = at + g;
+        uint32_t x = 0u;
+        if (g < kSufData && di < all) x = *(di < n ? k + di : v + (di - n));
+        if (g == (uint32_t)SUF_WORD_NEXT) x = after;
+        b[8 * q] = x;
       }
-      __syncwarp();
+      cur = after;
     }
   }
 }
@@ -497,13 +539,14 @@ MT_DEV void lane_retire_chain(const pool_view& p, uint32_t head) {
   const uint32_t hdr = ld_relaxed_u32(p.addr(head) + SUF_WORD_HDR);
   const uint32_t nn = suf_nodes(hdr & kMaxLen16, hdr >> 16);
   uint32_t c = head;
+#pragma unroll 1
   for (uint32_t q = 0; q < nn; ++q) {
     if (!p.valid(c)) break;
     const uint32_t nx = ld_relaxed_u32(p.addr(c) + SUF_WORD_NEXT);
     retire_slab(p, c);
     c = nx;
   }
-  if (c != kInvalid) record_error(p, ERR_CORRUPT, MT_AT(SRC_LANE));
+  if (c != kInvalid) lane_error(p.err, ERR_CORRUPT, MT_AT(SRC_LANE));
 }
 
 // x = v where c holds, as a select: a conditional store would make the compiler
@@ -543,44 +586,70 @@ MT_DEV void lane_remove_entry(uint32_t (&w)[32], uint32_t pos) {
   w[WORD_KS] = (ks & low) | ((ks >> 2) & ~low);
   w[WORD_META] -= 1u;
 }
-// Publish the edited image of a locked node; the stored meta keeps LOCK set.
-MT_DEV void lane_publish_locked(const pool_view& p, uint32_t idx, uint32_t (&w)[32]) {
-  w[WORD_META] = (w[WORD_META] | META_LOCK) + META_VERSION_ONE;
-  w[WORD_CSUM] = lane_checksum(w);
-  lane_store_weak(p.addr(idx), w);
+// Where a full border node is cut: 6 or 7, never between the two entries of
+// one slice.  high: the largest slice of the lower half.
+MT_DEV uint32_t lane_split_pos(const uint32_t (&w)[32], uint32_t& high) {
+  constexpr int h = kMaxEntries / 2;
+  const uint32_t k5 = w[2 * (h - 1)], k6 = w[2 * h];
+  high = k5;  // where the cut moves up, entry h has the same slice
+  return k5 == k6 ? h + 1 : h;
 }
-
-// Write the upper half of the full border node w (entries sp.., sp 6 or 7) to
-// slab R as a new node, with the new entry at position pos of the old order
-// (pos >= sp) when it belongs there.
-MT_DEV void lane_store_right_half(const pool_view& p, uint32_t R, const uint32_t (&w)[32], uint32_t sp, bool with_new,
-                                  uint32_t pos, uint32_t key, uint32_t val, uint32_t state) {
-  uint32_t r[32];
-  const uint32_t cnt = (uint32_t)kMaxEntries - sp;
-  const bool seven = sp == 7u;
-  // Entries 0..6 of the half (at most 7), then the new one shifted in.
+// The image of the upper half (entries sp..) as a node of its own.
+MT_DEV void lane_upper_half(uint32_t (&w)[32], uint32_t sp) {
+  const bool up = sp == (uint32_t)kMaxEntries / 2u + 1u;
+  constexpr int h = kMaxEntries / 2;
 #pragma unroll
-  for (int k = 14; k < 28; ++k) r[k] = 0u;
-#pragma unroll
-  for (int e = 0; e < 7; ++e) {
+  for (int e = 0; e < kMaxEntries; ++e) {
     // (By value: a conditional over array elements would index the array.)
-    const uint32_t k6 = w[2 * (e + 6)], v6 = w[2 * (e + 6) + 1];
-    const uint32_t k7 = e + 7 < kMaxEntries ? w[2 * (e + 7 < kMaxEntries ? e + 7 : 0)] : 0u;
-    const uint32_t v7 = e + 7 < kMaxEntries ? w[2 * (e + 7 < kMaxEntries ? e + 7 : 0) + 1] : 0u;
-    r[2 * e] = seven ? k7 : k6;
-    r[2 * e + 1] = seven ? v7 : v6;
+    const uint32_t ka = e + h < kMaxEntries ? w[2 * (e + h < kMaxEntries ? e + h : 0)] : 0u;
+    const uint32_t va = e + h < kMaxEntries ? w[2 * (e + h < kMaxEntries ? e + h : 0) + 1] : 0u;
+    const uint32_t kb = e + h + 1 < kMaxEntries ? w[2 * (e + h + 1 < kMaxEntries ? e + h + 1 : 0)] : 0u;
+    const uint32_t vb = e + h + 1 < kMaxEntries ? w[2 * (e + h + 1 < kMaxEntries ? e + h + 1 : 0) + 1] : 0u;
+    w[2 * e] = up ? kb : ka;
+    w[2 * e + 1] = up ? vb : va;
   }
-  r[WORD_HIGH] = w[WORD_HIGH];
-  r[WORD_SIB] = w[WORD_SIB];
-  r[WORD_META] = META_BORDER | (w[WORD_META] & META_SIB) | cnt;
-  r[WORD_KS] = w[WORD_KS] >> (2u * sp);
-  if (with_new) lane_insert_entry(r, pos - sp, key, val, state);
-  r[WORD_CSUM] = lane_checksum(r);
-  lane_store_weak(p.addr(R), r);
+  w[WORD_META] = META_BORDER | (w[WORD_META] & META_SIB) | ((uint32_t)kMaxEntries - sp);
+  w[WORD_KS] >>= 2u * sp;
+}
+// The image of the lower half (entries 0 .. sp-1), with its new sibling.
+MT_DEV void lane_lower_half(uint32_t (&w)[32], uint32_t sp, uint32_t high, uint32_t sib) {
+#pragma unroll
+  for (int e = kMaxEntries / 2; e < kMaxEntries; ++e) {
+    lane_set_if((uint32_t)e >= sp, w[2 * e], 0u);
+    lane_set_if((uint32_t)e >= sp, w[2 * e + 1], 0u);
+  }
+  w[WORD_KS] &= (1u << (2u * sp)) - 1u;
+  w[WORD_META] = (w[WORD_META] & ~META_COUNT) | META_SIB | sp;
+  w[WORD_HIGH] = high;
+  w[WORD_SIB] = sib;
 }
 
 // What a lane has to do at its border node.
 enum lane_job : uint32_t { JOB_NONE = 0, JOB_ADD = 1, JOB_SET = 2, JOB_DEL = 3 };
+
+// The call's logs of sparse nodes and emptied layers (as coop_erase).
+MT_DEV void lane_log_erase(const tree_view& tv, const lane_place& at, const uint32_t* key, uint32_t slice,
+                           uint32_t meta) {
+  const uint32_t left = meta & META_COUNT;
+  const bool is_root = (meta & META_ROOT) != 0u;
+  if (tv.merge_log != nullptr && !is_root && (left == kMergeAt || left == 0u)) {
+    const uint32_t r = atomicAdd(tv.merge_log, 1u);
+    if (r < tv.merge_cap) {
+      tv.merge_log[2u + 2u * r] = at.root;
+      tv.merge_log[3u + 2u * r] = slice;
+    }
+  }
+  if (tv.layer_log != nullptr && at.layer >= 1u && at.layer < kLayerRecWords && left == 0u && !(meta & META_SIB) &&
+      (is_root || tv.merge_log != nullptr)) {
+    const uint32_t r = atomicAdd(tv.layer_log, 1u);
+    if (r < tv.layer_cap) {
+      uint32_t* rec = tv.layer_log + 2u + (size_t)kLayerRecWords * r;
+      rec[0] = at.layer;
+#pragma unroll 1
+      for (uint32_t q = 0; q < at.layer; ++q) rec[1u + q] = key[q];
+    }
+  }
+}
 
 struct defer_list {
   uint32_t* list;   // requests handed to the tile kernel
@@ -619,6 +688,7 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
   const pool_view& p = tv.pool;
   const uint32_t per = max(1u, min(32u, (a.n + warps - 1u) / warps));
   uint32_t shard = (warp * 0x9E3779B1u) % p.num_shards;
+#pragma unroll 1
   for (uint32_t base = warp * per; base < a.n; base += warps * per) {
     if (__any_sync(kAll, slot == 0u && fatal_error(p))) break;
     const uint32_t pos = base + slot;
@@ -633,7 +703,7 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
         vlen = a.value_lengths_in ? a.value_lengths_in[i] : a.max_value_length;
     }
     const bool bad = valid && (klen > a.max_key_length || vlen > a.max_value_length || kind > MT_REQ_UPDATE);
-    if (bad) record_error(p, ERR_INVALID_ARG);
+    if (bad) lane_error(p.err, ERR_INVALID_ARG, MT_AT(SRC_LANE));
     bool combined = false;
     if (kUpdates && valid && a.leader_of != nullptr) combined = a.leader_of[i] != kInvalid;
     const bool act = valid && !bad && !combined;
@@ -649,19 +719,19 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
 
     // 1. To the border node.
     lane_place at;
-    at.found = false;
-    at.layer = 0;
-    at.idx = at.parent = at.root = 0;
-    if (go && !lane_locate<true>(tv, key, klen, at)) go = false;
+    at.idx = 0;
+    at.full = false;
+    lane_locate<true>(tv, go, key, klen, at);
     bool chain = go && at.found && (at.state == KS_SUFFIX || (find && at.state == KS_LONGVAL));
     if (chain && !p.valid(at.val)) {
-      record_error(p, ERR_CORRUPT, MT_AT(SRC_LANE));
+      lane_error(p.err, ERR_CORRUPT, MT_AT(SRC_LANE));
       chain = go = false;
     }
 
     // 2. Chains: compare and copy, then write.
     const bool more = at.layer + 1u < klen;
     const uint32_t rest = more ? klen - at.layer - 1u : 0u;
+    if (chain) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.addr(at.val)));
     bool eq = false;
     uint32_t cv = 0, res = 0, found_len = 0;
     warp_chains<kFinds>(p, chain, at.val, key + at.layer + 1u, rest, find ? val : nullptr, a.max_value_length, eq, cv);
@@ -686,19 +756,22 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
         job = JOB_ADD;
       }
     }
-    uint32_t nv = kInvalid, ns = KS_VALUE;
+    uint32_t nv = kInvalid, ns = KS_VALUE, spare = kInvalid;
     if (kChains) {
       uint32_t need = 0;
+      const bool right_half = kInserts && job == JOB_ADD && at.full && at.parent != kInvalid;
       if (job == JOB_ADD || job == JOB_SET) {
         ns = more ? KS_SUFFIX : (vlen == 1u ? KS_VALUE : KS_LONGVAL);
         if (ns == KS_VALUE) nv = val[0];
         else need = suf_nodes(rest, vlen);
       }
       lane_slabs sl{};
-      if (!warp_take_slabs(p, need, shard, sl)) {
+      if (!warp_take_slabs(p, need + (right_half ? 1u : 0u), shard, sl)) {
         job = JOB_NONE;
         defer = true;
         need = 0;
+      } else if (right_half) {
+        spare = lane_slab(p, sl, need);
       }
       warp_write_chains(p, need != 0u, sl, key + at.layer + 1u, rest, val, vlen, nv);
       __syncwarp();
@@ -707,48 +780,40 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
 
     // 3. The border node.
     const uint32_t slice = klen > 0u && act ? key[at.layer] : 0u;
-    uint32_t idx = at.idx, tries = 0, spare = kInvalid, old_chain = kInvalid;
-    bool want_spare = false;
+    uint32_t idx = at.idx, tries = 0, old_chain = kInvalid;
+#pragma unroll 1
     while (__any_sync(kAll, job != JOB_NONE)) {
-      if (kInserts && __any_sync(kAll, want_spare && spare == kInvalid)) {
-        lane_slabs sl{};
-        const uint32_t need = want_spare && spare == kInvalid ? 1u : 0u;
-        if (warp_take_slabs(p, need, shard, sl)) {
-          if (need) spare = lane_slab(p, sl, 0u);
-        } else {
-          job = JOB_NONE;
-          defer = true;
-          want_spare = false;
-        }
-      }
       uint32_t w[32];
-      bool won = false, split = false;
-      uint32_t pslot = 0, e = 0, st = 0, sp = 0;
-      if (job != JOB_NONE) {
-        uint32_t pmeta = 0;
-        bool parent_ok = true;
-        if (++tries > kLaneTries) {
-          job = JOB_NONE;
-          defer = true;
-        }
-        if (kInserts && job != JOB_NONE && want_spare) {
-          // The node was full: its parent must list it and have room.
-          parent_ok = lane_read_fresh(p, at.parent, w);
-          pmeta = w[WORD_META];
-          uint32_t hits = 0;
+      bool won = false, split = false, parent_ok = false;
+      uint32_t e = 0, pslot = 0, pmeta = 0;
+      if (job != JOB_NONE && ++tries > kLaneTries) {
+        job = JOB_NONE;
+        defer = true;
+      }
+      // Where the node is to be split, its parent must list it and have room;
+      // then the node itself.  A torn image counts as a lock that is held.
+      if (kInserts && job != JOB_NONE && spare != kInvalid) {
+        lane_load_relaxed(p.addr(at.parent), w);
+        pmeta = lane_verify(w) ? w[WORD_META] : META_LOCK;
+        uint32_t hits = 0;
 #pragma unroll
-          for (int k = 0; k < kMaxEntries; ++k)
-            if ((uint32_t)k < (pmeta & META_COUNT) && w[2 * k + 1] == idx) hits |= 1u << k;
-          parent_ok = parent_ok && hits != 0u && !(pmeta & META_BORDER) && (pmeta & META_COUNT) < (uint32_t)kMaxEntries;
-          pslot = hits ? (uint32_t)__ffs(hits) - 1u : 0u;
-        }
-        if (job != JOB_NONE && !lane_read_fresh(p, idx, w)) job = JOB_NONE;  // error recorded
+        for (int k = 0; k < kMaxEntries; ++k)
+          if ((uint32_t)k < (pmeta & META_COUNT) && w[2 * k + 1] == idx) hits |= 1u << k;
+        parent_ok = (pmeta & META_LOCK) ||
+                    (hits != 0u && !(pmeta & META_BORDER) && (pmeta & META_COUNT) < (uint32_t)kMaxEntries);
+        pslot = (uint32_t)__ffs(hits) - 1u;
+      }
+      bool read = false;
+      if (job != JOB_NONE) {
+        lane_load_relaxed(p.addr(idx), w);
+        read = lane_verify(w);
+      }
+      if (read) {
         const uint32_t meta = w[WORD_META];
-        if (job == JOB_NONE) {
-        } else if ((meta & META_SIB) && slice > w[WORD_HIGH]) {
+        if ((meta & META_SIB) && slice > w[WORD_HIGH]) {
           idx = w[WORD_SIB];
           if (!p.valid(idx)) {
-            record_error(p, ERR_CORRUPT, MT_AT(SRC_LANE));
+            lane_error(p.err, ERR_CORRUPT, MT_AT(SRC_LANE));
             job = JOB_NONE;
           }
         } else if (!(meta & META_BORDER)) {
@@ -756,32 +821,18 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
           defer = true;
         } else if (!(meta & META_LOCK)) {
           const uint32_t ks = w[WORD_KS];
-          const uint32_t okm = lane_eligible(meta, ks, more);
-          uint32_t hit = 0, v = 0, before = 0;
-#pragma unroll
-          for (int k = 0; k < kMaxEntries; ++k) {
-            if ((uint32_t)k < (meta & META_COUNT) &&
-                (w[2 * k] < slice || (more && w[2 * k] == slice && !(ks & (1u << (2 * k))))))
-              ++before;
-            if (w[2 * k] == slice && (okm & (1u << (2 * k)))) {
-              hit = 1u << (2 * k);
-              v = w[2 * k + 1];
-            }
-          }
-          st = (more ? KS_MORE : 0u) | ((ks & (hit << 1)) ? KS_SLAB : 0u);
-          e = before;  // entries before it: the entry's own position if there is one
+          uint32_t k, v;
+          e = lane_search(w, slice, more, k, v);
+          const bool hit = lane_is_entry(meta, ks, e, k, slice, more);
+          const uint32_t st = ks_get(ks, e);
           bool lock = false;
           if (job == JOB_ADD) {
-            if (hit) {
-              job = JOB_NONE;  // the slice was taken meanwhile
+            const bool full = (meta & META_COUNT) >= (uint32_t)kMaxEntries;
+            if (hit || (full && ((meta & META_ROOT) || !parent_ok))) {
+              job = JOB_NONE;  // the slice was taken meanwhile, or a split that is not this node's alone
               defer = true;
-            } else if ((meta & META_COUNT) < (uint32_t)kMaxEntries) {
+            } else if (!full) {
               lock = true;
-            } else if ((meta & META_ROOT) || at.parent == kInvalid || !parent_ok) {
-              job = JOB_NONE;
-              defer = true;
-            } else if (spare == kInvalid) {
-              want_spare = true;
             } else if (!(pmeta & META_LOCK)) {
               lock = split = true;
             }
@@ -809,87 +860,64 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
                 won = false;
               }
             }
-            if (won && job != JOB_ADD && (st & KS_SLAB)) old_chain = v;
+            if (won && job != JOB_ADD && (st & KS_SLAB)) old_chain = v;  // (not a LINK)
           }
         }
       }
-      if (kInserts && __any_sync(kAll, won && split)) {
+      // Publish: first new right halves (visible before anything leads to
+      // them), then the nodes, then the parents of split ones.
+      const bool splits = kInserts && __any_sync(kAll, won && split);
+      uint32_t high = 0;
+      if (splits) {
         if (won && split) {
-          // Never part the two entries of one slice.
-          sp = w[2 * (kMaxEntries / 2 - 1)] == w[2 * (kMaxEntries / 2)] ? kMaxEntries / 2 + 1 : kMaxEntries / 2;
-          const uint32_t h6 = w[10], h7 = w[12];
-          const uint32_t left_high = sp == 7u ? h7 : h6;
-          lane_store_right_half(p, spare, w, sp, slice > left_high, e, slice, nv, ns);
+          const uint32_t sp = lane_split_pos(w, high);
+          lane_upper_half(w, sp);
+          if (slice > high) lane_insert_entry(w, e - sp, slice, nv, ns);
+          lane_seal(w);
+          lane_store_weak(p.addr(spare), w);
+          lane_load_relaxed(p.addr(idx), w);  // locked by this lane: as read above
+          lane_lower_half(w, sp, high, spare);
         }
         __syncwarp();
         fence_release();
       }
       if (won) {
-        if (kInserts && split) {
-          const uint32_t h6 = w[10], h7 = w[12];
-          const uint32_t left_high = sp == 7u ? h7 : h6;
+        if (kInserts && job == JOB_ADD && (!split || slice <= high)) lane_insert_entry(w, e, slice, nv, ns);
+        if (kChains && job == JOB_SET) {
 #pragma unroll
-          for (int k = 6; k < kMaxEntries; ++k)
-            if ((uint32_t)k >= sp) w[2 * k] = w[2 * k + 1] = 0u;
-          w[WORD_KS] &= (1u << (2u * sp)) - 1u;
-          w[WORD_META] = (w[WORD_META] & ~META_COUNT) | META_SIB | sp;
-          w[WORD_HIGH] = left_high;
-          w[WORD_SIB] = spare;
-          if (slice <= left_high) lane_insert_entry(w, e, slice, nv, ns);
-          lane_publish_locked(p, idx, w);
-          lane_load_relaxed(p.addr(at.parent), w);  // locked: as read above
-          lane_insert_entry(w, pslot, left_high, idx, 0u);
-#pragma unroll
-          for (int k = 1; k < kMaxEntries; ++k)
-            lane_set_if((uint32_t)k == pslot + 1u, w[2 * k + 1], spare);
-          lane_publish_locked(p, at.parent, w);
-          spare = kInvalid;
-        } else {
-          if (job == JOB_ADD) {
-            lane_insert_entry(w, e, slice, nv, ns);
-          } else if (job == JOB_SET) {
-#pragma unroll
-            for (int k = 0; k < kMaxEntries; ++k)
-              lane_set_if((uint32_t)k == e, w[2 * k + 1], nv);
-            w[WORD_KS] = (w[WORD_KS] & ~(3u << (2u * e))) | (ns << (2u * e));
-          } else {
-            lane_remove_entry(w, e);
-          }
-          lane_publish_locked(p, idx, w);
+          for (int k = 0; k < kMaxEntries; ++k) lane_set_if((uint32_t)k == e, w[2 * k + 1], nv);
+          w[WORD_KS] = (w[WORD_KS] & ~(3u << (2u * e))) | (ns << (2u * e));
         }
+        if (kErases && job == JOB_DEL) lane_remove_entry(w, e);
+        w[WORD_META] = (w[WORD_META] | META_LOCK) + META_VERSION_ONE;
+        lane_seal(w);
+        lane_store_weak(p.addr(idx), w);
+      }
+      if (splits && won && split) {
+        lane_load_relaxed(p.addr(at.parent), w);  // locked by this lane: as read above
+        lane_insert_entry(w, pslot, high, idx, 0u);
+#pragma unroll
+        for (int k = 1; k < kMaxEntries; ++k) lane_set_if((uint32_t)k == pslot + 1u, w[2 * k + 1], spare);
+        w[WORD_META] = (w[WORD_META] | META_LOCK) + META_VERSION_ONE;
+        lane_seal(w);
+        lane_store_weak(p.addr(at.parent), w);
       }
       if (__any_sync(kAll, won)) fence_release();
       if (won) {
         red_and_relaxed(p.addr(idx) + WORD_META, ~META_LOCK);
-        if (kInserts && split) red_and_relaxed(p.addr(at.parent) + WORD_META, ~META_LOCK);
-        if (kErases && job == JOB_DEL) {
-          const uint32_t left = w[WORD_META] & META_COUNT;
-          const bool is_root = (w[WORD_META] & META_ROOT) != 0u;
-          if (tv.merge_log != nullptr && !is_root && (left == kMergeAt || left == 0u)) {
-            const uint32_t r = atomicAdd(tv.merge_log, 1u);
-            if (r < tv.merge_cap) {
-              tv.merge_log[2u + 2u * r] = at.root;
-              tv.merge_log[3u + 2u * r] = slice;
-            }
-          }
-          if (tv.layer_log != nullptr && at.layer >= 1u && at.layer < kLayerRecWords && left == 0u &&
-              !(w[WORD_META] & META_SIB) && (is_root || tv.merge_log != nullptr)) {
-            const uint32_t r = atomicAdd(tv.layer_log, 1u);
-            if (r < tv.layer_cap) {
-              uint32_t* rec = tv.layer_log + 2u + (size_t)kLayerRecWords * r;
-              rec[0] = at.layer;
-              for (uint32_t q = 0; q < at.layer; ++q) rec[1u + q] = key[q];
-            }
-          }
+        if (kInserts && split) {
+          red_and_relaxed(p.addr(at.parent) + WORD_META, ~META_LOCK);
+          spare = kInvalid;
         }
-        if (old_chain != kInvalid) lane_retire_chain(p, old_chain);
+        if (kErases && job == JOB_DEL) lane_log_erase(tv, at, key, slice, w[WORD_META]);
         nv = kInvalid;  // in the tree now
         res = 1u;
         job = JOB_NONE;
       }
     }
-    // Slabs taken in vain.
-    if (kChains && nv != kInvalid && (ns & KS_SLAB)) lane_retire_chain(p, nv);
+    // Chains replaced or erased, and slabs taken in vain.
+    if (kChains && (ns & KS_SLAB) && nv != kInvalid) old_chain = nv;
+    if (old_chain != kInvalid) lane_retire_chain(p, old_chain);
     if (kInserts && spare != kInvalid) retire_slab(p, spare);
 
     // 4. Results, and the requests left to the tile kernel.

@@ -5,8 +5,7 @@
 //                   border node  : value = inline value / suffix slab / layer root
 //                   interior node: key = separator (largest slice routed to the
 //                                  child), value = child slab
-//   word 26       : checksum of the other 31 words (LOCK bit masked)
-//   word 27       : reserved (0)
+//   words 26, 27  : 64-bit checksum of the other 30 words (LOCK bit masked), low half first
 //   word 28       : high key (largest slice this node covers; 0xFFFFFFFF for the
 //                   rightmost node of a level)
 //   word 29       : right sibling slab (valid iff META_SIB)
@@ -57,23 +56,36 @@ constexpr uint32_t META_VERSION_ONE = 1u << 16;
 
 constexpr int WORD_CSUM = 26, WORD_HIGH = 28, WORD_SIB = 29, WORD_META = 30, WORD_KS = 31;
 
-// Contribution of word g (value v) to a node checksum: a bijection of v for
-// every position (xor with a position constant, multiply by an odd constant,
-// xor-shift), so a torn image differing from a published one in a single word
-// always fails, and one differing in several words passes only if their mixed
-// differences cancel exactly modulo 2^32.  (One multiply per word: the
-// verification runs on every lock-free node load.)
-MT_HD uint32_t csum_term(uint32_t g, uint32_t v) {
-  if (g == (uint32_t)WORD_CSUM) return 0u;
-  if (g == (uint32_t)WORD_META) v &= ~(1u << 4);  // LOCK bit changes without a republish
-  const uint32_t x = (v ^ (g * 0x9E3779B9u) ^ 0x5BD1E995u) * 0x7FEB352Du;
-  return x ^ (x >> 15);
+// A node's checksum is the sum over its other words of word times a 32-bit odd
+// constant of the word's position, modulo 2^64, plus a constant (so that a
+// cleared slab is not an image).  A torn image that differs from a published
+// one in one word always fails (the difference is below 2^64 and not 0); one
+// that differs in several words passes only if the products of the differences
+// and the positions' constants cancel modulo 2^64.  One multiply-add per word:
+// the verification runs on every lock-free node load.  (The 32-bit form before
+// it, a multiply and an xor-shift per word, took five instructions a word: 155
+// of about 300 per node visit of a lane.)
+constexpr uint64_t kCsumInit = 0x5BD1E9955BD1E995ull;
+MT_HD uint32_t csum_factor(uint32_t g) {
+  const uint32_t x = (2u * g + 1u) * 0x9E3779B1u;
+  return (x ^ (x >> 15)) | 1u;
 }
-// Host/device checksum of a full 32-word node image.
-MT_HD uint32_t node_checksum(const uint32_t* w) {
-  uint32_t h = 0;
+MT_HD uint64_t csum_term(uint32_t g, uint32_t v) {
+  if (g == (uint32_t)WORD_CSUM || g == (uint32_t)WORD_CSUM + 1u) return 0u;
+  if (g == (uint32_t)WORD_META) v &= ~(1u << 4);  // LOCK bit changes without a republish
+  return (uint64_t)v * csum_factor(g);
+}
+// Host/device checksum of a full 32-word node image, and the one it carries.
+MT_HD uint64_t node_checksum(const uint32_t* w) {
+  uint64_t h = kCsumInit;
   for (uint32_t g = 0; g < 32u; ++g) h += csum_term(g, w[g]);
   return h;
+}
+MT_HD uint64_t stored_checksum(const uint32_t* w) { return (uint64_t)w[WORD_CSUM + 1] << 32 | w[WORD_CSUM]; }
+MT_HD void seal_image(uint32_t* w) {
+  const uint64_t h = node_checksum(w);
+  w[WORD_CSUM] = (uint32_t)h;
+  w[WORD_CSUM + 1] = (uint32_t)(h >> 32);
 }
 
 MT_HD uint32_t ks_get(uint32_t ks, uint32_t e) { return (ks >> (2u * e)) & 3u; }
@@ -148,14 +160,21 @@ struct node {
 #pragma unroll
     for (int k = 0; k < W; ++k) w[k] = 0u;
   }
-  MT_DEV uint32_t tile_checksum(const tile<T>& t) const {
-    uint32_t h = 0;
+  MT_DEV uint64_t tile_checksum(const tile<T>& t) const {
+    uint64_t h = 0;
 #pragma unroll
     for (int k = 0; k < W; ++k) h += csum_term(t.rank * W + k, w[k]);
-    return t.add_all(h);
+    // The 64-bit sum over the lanes from three 32-bit ones (no carry is lost).
+    const uint32_t a = t.add_all((uint32_t)h & 0xFFFFu), b = t.add_all((uint32_t)h >> 16);
+    const uint32_t c = t.add_all((uint32_t)(h >> 32));
+    return kCsumInit + a + ((uint64_t)b << 16) + ((uint64_t)c << 32);
   }
-  // Write the checksum word of the current image (call after encode_header).
-  MT_DEV void seal(const tile<T>& t) { set_word(t, WORD_CSUM, tile_checksum(t)); }
+  // Write the checksum words of the current image (call after encode_header).
+  MT_DEV void seal(const tile<T>& t) {
+    const uint64_t h = tile_checksum(t);
+    set_word(t, WORD_CSUM, (uint32_t)h);
+    set_word(t, WORD_CSUM + 1, (uint32_t)(h >> 32));
+  }
   // Load an image that concurrent writers may be publishing: reload until the
   // checksum matches (bounded), else record corruption.
   template <ld_order O>
@@ -163,7 +182,8 @@ struct node {
     for (uint32_t r = 0; r < kTornRetries; ++r) {
       load<O>(t, p, i);
       if constexpr (O == ld_order::NC) return true;
-      if (tile_checksum(t) == word(t, WORD_CSUM)) return true;
+      const uint32_t lo = word(t, WORD_CSUM), hi = word(t, WORD_CSUM + 1);
+      if (tile_checksum(t) == ((uint64_t)hi << 32 | lo)) return true;
     }
     if (t.leader()) record_error(p, ERR_CORRUPT, MT_AT(SRC_NODE));
     return false;
