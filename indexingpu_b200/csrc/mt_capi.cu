@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "mt_lane.cuh"
+#include "mt_scan.cuh"
 
 namespace mtb {
 
@@ -135,8 +136,9 @@ __global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) lane_kernel(tree
   lane_serve<OP>(tv, a, dl);
 }
 
-template <int T, bool CONC>
-__global__ void __launch_bounds__(kBlock, MT_MIN_BLOCKS_PER_SM) scan_kernel(tree_view tv, scan_args a) {
+template <bool CONC>
+__global__ void __launch_bounds__(kBlock, MT_SCAN_BLOCKS) scan_kernel(tree_view tv, scan_args a) {
+  constexpr int T = 16;
   tile<T> t;
   const uint32_t tile_id = (blockIdx.x * blockDim.x + threadIdx.x) / T;
   const uint32_t num_tiles = (gridDim.x * blockDim.x) / T;
@@ -175,8 +177,9 @@ __global__ void __launch_bounds__(kBlock, MT_MIN_BLOCKS_PER_SM) scan_kernel(tree
       o.maxK = a.max_key_length;
       const uint32_t* lower = a.lower + (size_t)q * a.max_key_length;
       const uint32_t* upper = a.upper ? a.upper + (size_t)q * a.max_key_length : nullptr;
-      const uint32_t c = coop_scan<T, CONC>(t, tv, lower, ll, a.use_upper != 0u && upper != nullptr, upper, ul,
-                                           a.max_count, o, frames);
+      const uint32_t c = scan_query<CONC>(t, tv, lower, ll, a.use_upper != 0u && upper != nullptr, upper, ul,
+                                          a.max_count, o, frames);
+      if (frames.cur != kInvalid) frames.release(t, tv.pool);
       if (t.rank == r) cnt = c;
     }
     if (valid && a.counts) a.counts[i] = cnt;
@@ -461,11 +464,10 @@ int launch_mixed(mt_masstree* t, batch_args a, cudaStream_t s) {
   return rc;
 }
 
-template <int T, bool CONC>
-int launch_scan_t(mt_masstree* t, scan_args a, cudaStream_t s) {
-  const void* fn = (const void*)scan_kernel<T, CONC>;
-  const int grid = grid_for(t, fn);
-  const size_t tiles = (size_t)grid * kBlock / T;
+template <bool CONC>
+int launch_scan(mt_masstree* t, scan_args a, cudaStream_t s) {
+  const int grid = grid_for(t, (const void*)scan_kernel<CONC>);
+  const size_t tiles = (size_t)grid * kBlock / 16;
   if (tiles > t->frames_tiles) {
     // Scan frames: grown on demand, kept for later calls.
     cudaStreamSynchronize(s);
@@ -476,19 +478,8 @@ int launch_scan_t(mt_masstree* t, scan_args a, cudaStream_t s) {
     t->frames_tiles = tiles;
   }
   a.frames = t->frames;
-  scan_kernel<T, CONC><<<grid, kBlock, 0, s>>>(t->tv, a);
+  scan_kernel<CONC><<<grid, kBlock, 0, s>>>(t->tv, a);
   return cuda_status(cudaGetLastError());
-}
-
-template <bool CONC>
-int launch_scan(mt_masstree* t, const scan_args& a, cudaStream_t s) {
-  switch (t->scan_tile_size ? t->scan_tile_size : t->tile_size) {
-    case 4: return launch_scan_t<4, CONC>(t, a, s);
-    case 8: return launch_scan_t<8, CONC>(t, a, s);
-    case 16: return launch_scan_t<16, CONC>(t, a, s);
-    case 32: return launch_scan_t<32, CONC>(t, a, s);
-    default: return MT_ERR_INVALID_ARG;
-  }
 }
 
 bool valid_tile(uint32_t ts) { return host_valid_tile(ts); }
@@ -515,8 +506,9 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
   const size_t stack_bytes = nslabs * 4u;
   const size_t ctr_bytes = (size_t)kShards * 3u * kCtrStride * sizeof(int);
   const size_t err_bytes = 128;
-  // The defer list of the lane kernels: 1/256 of the pool, at most 1M entries.
-  const uint64_t defer_cap = std::min<uint64_t>(1u << 20, std::max<uint64_t>(4096u, pool_bytes / 1024u));
+  // The defer list of the lane kernels: 1/256 of the pool, at most 16M entries
+  // (a call of more requests is served in pieces, each with its own tail).
+  const uint64_t defer_cap = std::min<uint64_t>(1u << 24, std::max<uint64_t>(4096u, pool_bytes / 1024u));
   const size_t total = slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes + 128 + defer_cap * 4u;
   if (cudaMalloc(&t->mem, total) != cudaSuccess) { delete t; return MT_ERR_OOM; }
   char* base = (char*)t->mem;

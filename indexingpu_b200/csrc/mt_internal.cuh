@@ -25,6 +25,9 @@ constexpr uint32_t kClassBarrierMin = 1u << 17;
 #ifndef MT_CHAIN_ROUND
 #define MT_CHAIN_ROUND 1  // chains in flight per eight lanes in the lane kernels
 #endif
+#ifndef MT_SCAN_BLOCKS
+#define MT_SCAN_BLOCKS 8
+#endif
 #ifndef MT_LANE_WRITE_BLOCKS
 #define MT_LANE_WRITE_BLOCKS 4  // and for the write and mixed kernels (an image, an edit and a fence: 128 registers)
 #endif

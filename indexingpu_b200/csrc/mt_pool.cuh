@@ -63,7 +63,7 @@ struct pool_view {
 // Where an error was detected: a source file number (high 16 bits) and line.
 #define MT_AT(file) ((((uint32_t)(file)) << 16) | (uint32_t)__LINE__)
 enum mt_src_file : uint32_t { SRC_TREE = 1, SRC_NODE = 2, SRC_SUFFIX = 3, SRC_POOL = 4, SRC_FIND = 5, SRC_CAPI = 6,
-                              SRC_MERGE = 7, SRC_BULK = 8, SRC_SERVE = 9, SRC_LANE = 10 };
+                              SRC_MERGE = 7, SRC_BULK = 8, SRC_SERVE = 9, SRC_LANE = 10, SRC_SCAN = 11 };
 
 // err[0] = first error code, err[1] = error count, err[2] = fatal flag,
 // err[3] = where the first error was detected (MT_AT; 0 if not given).  A
