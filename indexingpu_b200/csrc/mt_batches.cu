@@ -9,11 +9,11 @@
 //      under (sub-batch, class) with class = find / insert / update+erase,
 //      optionally split into short and long keys (filled from the two ends of
 //      the class's index region, so each class is served short keys first);
-//   3. either (default) for every sub-batch its three batches_class_kernel
-//      launches side by side on forked streams, joined before the next
-//      sub-batch, or (MT_FLAG_PERSISTENT) batches_persistent_kernel: a
-//      cooperative grid walks the sub-batches in order with one grid barrier
-//      between sub-batches.
+//   3. (MT_FLAG_PERSISTENT) batches_persistent_kernel: a cooperative grid walks
+//      the sub-batches in order with one grid barrier between sub-batches;
+//   or, by default, instead of 2 and 3: for every sub-batch one kernel that
+//      serves its requests one per lane (mt_lane.cuh), and a tile kernel for
+//      the few it hands on.
 // Sub-batch k+1 observes every effect of sub-batch k, as with one host call per
 // sub-batch; inside a sub-batch the classes have no order among each other
 // (as inside one mixed batch).  Nothing in the call allocates once
@@ -134,26 +134,36 @@ __global__ void __launch_bounds__(kBlock, MT_MIN_BLOCKS_PER_SM) batches_persiste
   wcache.release(tw, tv.pool);
 }
 
-// One class of one sub-batch (the forked form): the class kernels of a
-// sub-batch run side by side, each compiled for its class only.
-template <int T, int OP>
-__global__ void __launch_bounds__(kBlock, min_blocks_for<OP>) batches_class_kernel(tree_view tv, batches_view b,
-                                                                                     uint32_t sb) {
+// Default form: the requests of one sub-batch, one per lane, and then those
+// that the lanes handed on (their list is the sub-batch's part of lists, its
+// count the first of the sub-batch's counters).
+MT_DEV batch_args subbatch_args(const batches_view& b, uint32_t sb) {
+  batch_args a = class_args(b, sb, 0u);
+  a.index = nullptr;
+  a.n_dev = a.n_back_dev = nullptr;
+  a.n = a.region;
+  return a;
+}
+__global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) batches_lane_kernel(tree_view tv, batches_view b,
+                                                                                    uint32_t sb) {
   if (b.status[0]) return;
-  constexpr uint32_t cls = OP == OP_PASS_INSERT ? 1u : 2u;
+  const defer_list dl{b.lists + b.offsets[sb], b.counts + sb * kCountStride};
+  lane_serve<OP_MIXED, true>(tv, batch_source{subbatch_args(b, sb)}, dl);
+}
+template <int T>
+__global__ void __launch_bounds__(kBlock, MT_MIN_BLOCKS_PER_SM) batches_rest_kernel(tree_view tv, batches_view b,
+                                                                                    uint32_t sb) {
+  if (b.status[0]) return;
   tile<T> t;
   const uint32_t tile_id = (blockIdx.x * blockDim.x + threadIdx.x) / T;
   const uint32_t num_tiles = (gridDim.x * blockDim.x) / T;
   slab_cache<T> cache;
   cache.init(tv.pool, tile_id);
-  serve_requests<T, OP, true>(t, tv, cache, class_args(b, sb, cls), tile_id, num_tiles);
+  batch_args a = subbatch_args(b, sb);
+  a.index = b.lists + b.offsets[sb];
+  a.n_dev = b.counts + sb * kCountStride;
+  serve_requests<T, OP_MIXED, true>(t, tv, cache, a, tile_id, num_tiles);
   cache.release(t, tv.pool);
-}
-
-__global__ void __launch_bounds__(kBlock, MT_LANE_FIND_BLOCKS) batches_find_kernel(tree_view tv, batches_view b,
-                                                                                   uint32_t sb) {
-  if (b.status[0]) return;
-  lane_find<true>(tv, class_args(b, sb, 0u));
 }
 
 }  // namespace mtb
@@ -162,44 +172,23 @@ using namespace mtb;
 
 namespace {
 
-// The sub-batches' sizes are on the device only: the grid fills the GPU.
-int launch_class_finds(mt_masstree* t, const batches_view& b, uint32_t sb, cudaStream_t s) {
-  batches_find_kernel<<<host_lane_grid(t, (const void*)batches_find_kernel, b.max_total), kBlock, 0, s>>>(t->tv, b, sb);
-  return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
-}
+int launch_status() { return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA; }
 
-template <int T, int OP>
-int launch_class(mt_masstree* t, const batches_view& b, uint32_t sb, cudaStream_t s) {
-  const void* fn = (const void*)batches_class_kernel<T, OP>;
-  int bps = host_max_blocks_per_sm(fn, kBlock, 0);
+template <int T>
+int launch_rest(mt_masstree* t, const batches_view& b, uint32_t sb, cudaStream_t s) {
+  int bps = host_max_blocks_per_sm((const void*)batches_rest_kernel<T>, kBlock, 0);
   if (t->blocks_per_sm > 0) bps = std::min<int>(bps, (int)t->blocks_per_sm);
-  batches_class_kernel<T, OP><<<std::max(bps, 1) * t->sms, kBlock, 0, s>>>(t->tv, b, sb);
-  return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
+  batches_rest_kernel<T><<<std::max(bps, 1) * t->sms, kBlock, 0, s>>>(t->tv, b, sb);
+  return launch_status();
 }
 
-template <int OP>
-int launch_class_tile(mt_masstree* t, uint32_t tile, const batches_view& b, uint32_t sb, cudaStream_t s) {
-  switch (tile) {
-    case 4: return launch_class<4, OP>(t, b, sb, s);
-    case 8: return launch_class<8, OP>(t, b, sb, s);
-    case 16: return launch_class<16, OP>(t, b, sb, s);
-    default: return launch_class<32, OP>(t, b, sb, s);
-  }
-}
-
-// Forked form: per sub-batch, the insert class on the caller's stream and the
-// find and update/erase classes on the tree's two side streams, joined before
-// the next sub-batch starts.
-int launch_forked(mt_masstree* t, const batches_view& b, cudaStream_t s) {
-  const uint32_t tw = t->write_tile_size <= 16 ? 16u : 32u;
-  const uint32_t tu = t->upderase_tile_size ? t->upderase_tile_size : tw;
+// The sub-batches' sizes are on the device only: the grids fill the GPU.
+int launch_each(mt_masstree* t, const batches_view& b, cudaStream_t s) {
+  const int grid = host_lane_grid(t, (const void*)batches_lane_kernel, b.max_total);
   for (uint32_t sb = 0; sb < b.nsub; ++sb) {
-    int rc = host_fork(t, s);
-    if (rc) return rc;
-    rc = launch_class_tile<OP_PASS_INSERT>(t, tw, b, sb, s);
-    if (!rc) rc = launch_class_finds(t, b, sb, t->side[0]);
-    if (!rc) rc = launch_class_tile<OP_PASS_UPDERASE>(t, tu, b, sb, t->side[1]);
-    rc = host_join(t, s, rc);
+    batches_lane_kernel<<<grid, kBlock, 0, s>>>(t->tv, b, sb);
+    int rc = launch_status();
+    if (!rc) rc = t->write_tile_size <= 16 ? launch_rest<16>(t, b, sb, s) : launch_rest<32>(t, b, sb, s);
     if (rc) return rc;
   }
   return MT_OK;
@@ -282,9 +271,9 @@ extern "C" int mt_mixed_batches(mt_masstree* t, const mt_subbatch* subbatches, u
     const int grc = launch_grouped(t, b, s);
     if (grc != kGroupedUnavailable) return grc;
   }
+  if (!(flags & MT_FLAG_PERSISTENT)) return launch_each(t, b, s);
   batches_partition_kernel<<<t->sms * 4, 256, 0, s>>>(b);
   if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
-  if (!(flags & MT_FLAG_PERSISTENT)) return launch_forked(t, b, s);
   switch (t->tile_size) {
     case 4: return launch_persistent_tf<4>(t, b, s);
     case 8: return launch_persistent_tf<8>(t, b, s);

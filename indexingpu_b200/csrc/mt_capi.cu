@@ -126,14 +126,14 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for<OP>) batch_kernel(tree_
 
 template <bool CONC>
 __global__ void __launch_bounds__(kBlock, MT_LANE_FIND_BLOCKS) find_kernel(tree_view tv, batch_args a) {
-  lane_find<CONC>(tv, a);
+  lane_serve<OP_FIND, CONC>(tv, batch_source{a}, defer_list{nullptr, nullptr});
 }
 
 // Inserts, updates, erases and mixed batches, one request per lane.  4M-key
 // and 16M-key trees: see lane_serve.
 template <int OP>
 __global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) lane_kernel(tree_view tv, batch_args a, defer_list dl) {
-  lane_serve<OP>(tv, a, dl);
+  lane_serve<OP, true>(tv, batch_source{a}, dl);
 }
 
 template <bool CONC>
@@ -264,33 +264,6 @@ int host_max_blocks_per_sm(const void* fn, int block, size_t smem) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, block, smem) != cudaSuccess || b <= 0) b = 1;
   return b;
 }
-// Make the tree's two side streams wait for the work queued so far on s.
-int host_fork(mt_masstree* t, cudaStream_t s) {
-  if (!t->ev_fork) {
-    bool ok = cudaEventCreateWithFlags(&t->ev_fork, cudaEventDisableTiming) == cudaSuccess;
-    for (int k = 0; k < 2 && ok; ++k)
-      ok = cudaStreamCreateWithFlags(&t->side[k], cudaStreamNonBlocking) == cudaSuccess &&
-           cudaEventCreateWithFlags(&t->ev_join[k], cudaEventDisableTiming) == cudaSuccess;
-    if (!ok) return MT_ERR_CUDA;
-  }
-  if (cudaEventRecord(t->ev_fork, s) != cudaSuccess) return MT_ERR_CUDA;
-  for (int k = 0; k < 2; ++k)
-    if (cudaStreamWaitEvent(t->side[k], t->ev_fork, 0) != cudaSuccess) return MT_ERR_CUDA;
-  return MT_OK;
-}
-
-// Make s wait for the side streams.  Called after a fork even when a launch
-// failed (rc != MT_OK, returned unchanged), so that the side streams never run
-// ahead of the caller's stream.
-int host_join(mt_masstree* t, cudaStream_t s, int rc) {
-  for (int k = 0; k < 2; ++k) {
-    if (cudaEventRecord(t->ev_join[k], t->side[k]) != cudaSuccess ||
-        cudaStreamWaitEvent(s, t->ev_join[k], 0) != cudaSuccess)
-      rc = rc ? rc : MT_ERR_CUDA;
-  }
-  return rc;
-}
-
 int host_launch_reclaim(mt_masstree* t, cudaStream_t s) {
   reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->defer_mem);
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
@@ -593,11 +566,6 @@ int mt_destroy(mt_masstree* t) {
   host_pipe_free(t);
   if (t->mem) cudaFree(t->mem);
   if (t->h_err) cudaFreeHost(t->h_err);
-  for (int k = 0; k < 2; ++k) {
-    if (t->side[k]) cudaStreamDestroy(t->side[k]);
-    if (t->ev_join[k]) cudaEventDestroy(t->ev_join[k]);
-  }
-  if (t->ev_fork) cudaEventDestroy(t->ev_fork);
   delete t;
   return MT_OK;
 }

@@ -30,7 +30,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
-#include "mt_internal.cuh"
+#include "mt_lane.cuh"
 
 namespace mtb {
 
@@ -79,10 +79,10 @@ struct grouped_view {
   uint32_t* act;             // [m] at a run head: final write (kGKeep none, kGAbsent erase, else insert/update id)
   uint32_t* vals;            // [m][max_value_length] at a run head: the value the tree held
   uint32_t* heads;           // run heads of keys touched more than once (count: counts[0])
-  uint32_t* singles;         // inserts on keys touched once (count: counts[1])
-  uint32_t* singles_ue;      // updates and erases on keys touched once (count: counts[4])
+  uint32_t* singles;         // requests on keys touched once (count: counts[1])
   uint32_t* serial;          // heads of runs served one by one (count: counts[2])
-  uint32_t* finds;           // finds on keys touched once (count: counts[3])
+  uint32_t* rest;            // singles left to the tile kernel (count: counts[3])
+  uint32_t* rest_heads;      // final writes left to the tile kernel (count: counts[4])
   uint32_t* counts;          // [5], zeroed at the start of the call
   unsigned long long hash_mask;  // bits of the key hash used (mt_set_group_hash_bits)
 };
@@ -102,16 +102,6 @@ MT_DEV greq group_req(const grouped_view& g, uint32_t id) {
   r.klen = r.d->key_lengths ? r.d->key_lengths[r.i] : g.b.max_key_length;
   r.vlen = (r.kind == MT_REQ_INSERT || r.kind == MT_REQ_UPDATE) ? r.d->value_lengths[r.i] : 0u;
   return r;
-}
-template <int T>
-MT_DEV greq greq_shfl(const tile<T>& t, const greq& r, int src) {
-  greq q;
-  q.d = reinterpret_cast<const mt_subbatch*>(t.shfl64(reinterpret_cast<uint64_t>(r.d), src));
-  q.i = t.shfl(r.i, src);
-  q.kind = t.shfl(r.kind, src);
-  q.klen = t.shfl(r.klen, src);
-  q.vlen = t.shfl(r.vlen, src);
-  return q;
 }
 // Warp-aggregated append of j to `list` (count at *count) by the lanes where want holds.
 MT_DEV void list_append(bool want, uint32_t* list, uint32_t* count, uint32_t j) {
@@ -216,100 +206,63 @@ __global__ void group_mark_kernel(grouped_view g) {
   }
 }
 
-// 4. Work lists: heads of keys touched more than once, writes and finds on
-// keys touched once.
+// 4. Work lists: heads of keys touched more than once, requests on keys
+// touched once.
 __global__ void group_list_kernel(grouped_view g) {
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x; base < g.m; base += stride) {
     const uint32_t j = base + threadIdx.x;
-    bool head = false, multi = false, ins = false, find = false;
+    bool head = false, multi = false;
     if (j < g.m && g.hash[j] < kGBad && g.pre[j].first == kGNoFirst && !(g.flags[j] & 1u)) {
       head = true;
       multi = !run_last(g, j);
-      ins = g.fn[j].a != kGAbsent;
-      find = !ins && g.fn[j].p == kGKeep;
     }
-    const bool single = head && !multi;
     list_append(head && multi, g.heads, &g.counts[0], j);
-    list_append(single && ins, g.singles, &g.counts[1], j);
-    list_append(single && !ins && !find, g.singles_ue, &g.counts[4], j);
-    list_append(single && find, g.finds, &g.counts[3], j);
+    list_append(head && !multi, g.singles, &g.counts[1], j);
   }
 }
 
-// Find that also tells a present key with an empty value from an absent one.
-template <int T>
-MT_DEV bool group_lookup(const tile<T>& t, const tree_view& tv, const uint32_t* key, uint32_t klen, uint32_t* out,
-                         uint32_t maxV, uint32_t& vlen) {
-  const pool_view& p = tv.pool;
-  uint32_t root = tv.root, hops = 0;
-  node<T> nd;
-  vlen = 0;
-  for (uint32_t layer = 0; layer < klen; ++layer) {
-    const uint32_t slice = key[layer];
-    const bool more = layer + 1u < klen;
-    if (!descend<T, kConc>(t, p, root, slice, nd, hops)) return false;
-    const int e = nd.match(t, slice, more);
-    if (e < 0) return false;
-    const uint32_t st = ks_get(nd.ks, (uint32_t)e);
-    const uint32_t v = nd.val_at(t, (uint32_t)e);
-    if (st == KS_LINK) { root = v; continue; }
-    if (st == KS_VALUE) {
-      if (maxV > 0u && t.leader()) out[0] = v;
-      vlen = 1u;
-      return true;
+// 5. The tree's state of the keys touched more than once (finds into g.vals;
+// present with an empty value is told from absent), and the requests on keys
+// touched once, one per lane.
+struct group_first_source {
+  grouped_view g;
+  MT_DEV uint32_t size() const { return g.counts[0] + g.counts[1]; }
+  MT_DEV uint32_t max_value_length() const { return g.b.max_value_length; }
+  template <int OP>
+  MT_DEV uint32_t fetch(const pool_view&, uint32_t pos, lane_request& r) const {
+    const uint32_t nh = g.counts[0];
+    const uint32_t j = pos < nh ? g.heads[pos] : g.singles[pos - nh];
+    const greq q = group_req(g, g.gid[j]);
+    r.id = j;
+    r.klen = q.klen;
+    r.key = greq_key(g, q);
+    if (pos < nh) {
+      r.kind = MT_REQ_FIND;
+      r.val = g.vals + (size_t)j * g.b.max_value_length;
+      return LANE_SERVE;
     }
-    if (!p.valid(v)) { if (t.leader()) record_error(p, ERR_CORRUPT, MT_AT(SRC_TREE)); return false; }
-    suffix_head<T> h;
-    h.template load<kConcSuffix>(t, p, v);
-    if (st == KS_SUFFIX) {
-      const uint32_t lk = klen - layer - 1u;
-      if (h.klen != lk) return false;
-      if (suffix_compare<T, kConcSuffix>(t, p, h, key + layer + 1u, lk).sign != 0) return false;
-    }
-    vlen = suffix_get_value<T, kConcSuffix>(t, p, h, out, maxV);
-    return true;
+    r.kind = q.kind;
+    r.vlen = q.vlen;
+    r.val = greq_val(g, q);
+    r.out_len = q.d->value_lengths + q.i;
+    r.out_ok = q.d->results ? q.d->results + q.i : nullptr;
+    return LANE_SERVE;
   }
-  return false;
-}
-
-// 5. Run heads of keys touched more than once: the tree's state of the key;
-// and the finds on keys touched once.
-template <int T>
-__global__ void __launch_bounds__(kBlock, MT_MIN_BLOCKS_PER_SM) group_head_kernel(tree_view tv, grouped_view g) {
-  tile<T> t;
-  const uint32_t tile_id = (blockIdx.x * blockDim.x + threadIdx.x) / T;
-  const uint32_t num_tiles = (gridDim.x * blockDim.x) / T;
-  const uint32_t maxV = g.b.max_value_length;
-  const uint32_t nh = g.counts[0], n = nh + g.counts[3];
-  // As in the batch kernels: each lane fetches one entry's request, then the
-  // tile serves the entries one after the other.
-  for (uint32_t base = tile_id * T; base < n; base += num_tiles * T) {
-    if (t.shfl((uint32_t)(t.leader() && fatal_error(tv.pool)), 0)) break;
-    const uint32_t mine = base + t.rank;
-    uint32_t j = 0;
-    greq rq{};
-    if (mine < n) {
-      j = mine < nh ? g.heads[mine] : g.finds[mine - nh];
-      rq = group_req(g, g.gid[j]);
-    }
-    const uint32_t cnt = min((uint32_t)T, n - base);
-    for (uint32_t q = 0; q < cnt; ++q) {
-      const greq r = greq_shfl(t, rq, (int)q);
-      const uint32_t jj = t.shfl(j, (int)q);
-      if (base + q >= nh) {  // a find on a key touched once: served directly
-        const uint32_t vo = coop_find<T, true>(t, tv, greq_key(g, r), r.klen, greq_val(g, r), maxV);
-        if (t.leader()) r.d->value_lengths[r.i] = vo;
-        continue;
-      }
-      uint32_t vl = 0;
-      const bool found = group_lookup<T>(t, tv, greq_key(g, r), r.klen, g.vals + (size_t)jj * maxV, maxV, vl);
-      if (t.leader()) {
-        g.init[jj] = found ? vl : kGAbsent;
-        g.act[jj] = kGKeep;
-      }
+  MT_DEV void found(uint32_t pos, const lane_request& r, bool present, uint32_t len) const {
+    if (pos < g.counts[0]) {
+      g.init[r.id] = present ? len : kGAbsent;
+      g.act[r.id] = kGKeep;
+    } else {
+      *r.out_len = len;
     }
   }
+  MT_DEV void result(uint32_t, const lane_request& r, bool ok) const {
+    if (r.out_ok != nullptr) *r.out_ok = ok;
+  }
+};
+__global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) group_first_kernel(tree_view tv, grouped_view g) {
+  lane_serve<OP_MIXED, true>(tv, group_first_source{g}, defer_list{g.rest, &g.counts[3]});
 }
 
 // 6. Results of the requests on keys touched more than once, from the scanned
@@ -352,61 +305,66 @@ __global__ void group_result_kernel(grouped_view g) {
   }
 }
 
-// 7. Writes: the requests on keys touched once, or the final write of every
-// key touched more than once.
-// MODE kGWInsert / kGWUpdErase: the inserts / the updates and erases on keys
-// touched once (they need nothing from the other passes and run beside them,
-// each kernel compiled for its kinds only); kGWHeads: the final writes.
-constexpr int kGWInsert = 0, kGWUpdErase = 1, kGWHeads = 2;
-template <int T, int MODE>
-__global__ void __launch_bounds__(kBlock, MT_WRITE_MIN_BLOCKS_PER_SM) group_write_kernel(tree_view tv, grouped_view g) {
+// 7. The final write of every key touched more than once, one per lane.
+struct group_final_source {
+  grouped_view g;
+  MT_DEV uint32_t size() const { return g.counts[0]; }
+  MT_DEV uint32_t max_value_length() const { return g.b.max_value_length; }
+  template <int OP>
+  MT_DEV uint32_t fetch(const pool_view&, uint32_t pos, lane_request& r) const {
+    const uint32_t j = g.heads[pos];
+    const uint32_t act = g.act[j];
+    if (act == kGKeep) return LANE_SKIP;
+    const greq q = group_req(g, g.gid[j]);
+    r.id = j;
+    r.klen = q.klen;
+    r.key = greq_key(g, q);
+    r.kind = MT_REQ_ERASE;
+    if (act != kGAbsent) {
+      const greq w = group_req(g, act);
+      r.kind = g.init[j] == kGAbsent ? MT_REQ_INSERT : MT_REQ_UPDATE;
+      r.vlen = w.vlen;
+      r.val = greq_val(g, w);
+    }
+    return LANE_SERVE;
+  }
+  MT_DEV void found(uint32_t, const lane_request&, bool, uint32_t) const {}
+  MT_DEV void result(uint32_t, const lane_request&, bool) const {}
+};
+__global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) group_final_kernel(tree_view tv, grouped_view g) {
+  lane_serve<OP_MIXED, true>(tv, group_final_source{g}, defer_list{g.rest_heads, &g.counts[4]});
+}
+
+// What the lanes handed on: HEADS, final writes, else requests on keys touched
+// once (never finds).
+template <int T, bool HEADS>
+__global__ void __launch_bounds__(kBlock, MT_WRITE_MIN_BLOCKS_PER_SM) group_rest_kernel(tree_view tv, grouped_view g) {
   tile<T> t;
   const uint32_t tile_id = (blockIdx.x * blockDim.x + threadIdx.x) / T;
   const uint32_t num_tiles = (gridDim.x * blockDim.x) / T;
   slab_cache<T> cache;
   cache.init(tv.pool, tile_id);
-  constexpr bool HEADS = MODE == kGWHeads;
-  const uint32_t n = HEADS ? g.counts[0] : (MODE == kGWInsert ? g.counts[1] : g.counts[4]);
-  for (uint32_t base = tile_id * T; base < n; base += num_tiles * T) {
+  const uint32_t n = g.counts[HEADS ? 4 : 3];
+  for (uint32_t k = tile_id; k < n; k += num_tiles) {
     if (t.shfl((uint32_t)(t.leader() && fatal_error(tv.pool)), 0)) break;
-    // Each lane fetches one entry: its request and, for a key touched more
-    // than once, the final write and the request whose value it writes.
-    const uint32_t mine = base + t.rank;
-    greq rq{}, wq{};
-    uint32_t act = kGKeep, init = kGAbsent;
-    if (mine < n) {
-      const uint32_t j = HEADS ? g.heads[mine] : (MODE == kGWInsert ? g.singles[mine] : g.singles_ue[mine]);
-      rq = group_req(g, g.gid[j]);
-      if (HEADS) {
-        act = g.act[j];
-        init = g.init[j];
-        if (act != kGKeep && act != kGAbsent) wq = group_req(g, act);
+    const uint32_t j = HEADS ? g.rest_heads[k] : g.rest[k];
+    const greq r = group_req(g, g.gid[j]);
+    const uint32_t* key = greq_key(g, r);
+    greq w = r;
+    uint32_t kind = r.kind;
+    if (HEADS) {
+      const uint32_t act = g.act[j];
+      kind = MT_REQ_ERASE;
+      if (act != kGAbsent) {
+        w = group_req(g, act);
+        kind = g.init[j] == kGAbsent ? MT_REQ_INSERT : MT_REQ_UPDATE;
       }
     }
-    const uint32_t cnt = min((uint32_t)T, n - base);
-    for (uint32_t q = 0; q < cnt; ++q) {
-      const greq r = greq_shfl(t, rq, (int)q);
-      const uint32_t* key = greq_key(g, r);
-      if constexpr (MODE == kGWInsert) {
-        const int res = coop_insert<T, false>(t, tv, cache, key, r.klen, greq_val(g, r), r.vlen);
-        if (t.leader() && r.d->results) r.d->results[r.i] = res == RES_OK;
-      } else if constexpr (MODE == kGWUpdErase) {
-        int res;
-        if (r.kind == MT_REQ_UPDATE) res = coop_update<T>(t, tv, cache, key, r.klen, greq_val(g, r), r.vlen);
-        else res = coop_erase<T>(t, tv, key, r.klen);
-        if (t.leader() && r.d->results) r.d->results[r.i] = res == RES_OK;
-      } else {
-        const uint32_t a = t.shfl(act, (int)q);
-        if (a == kGKeep) continue;
-        if (a == kGAbsent) {
-          coop_erase<T>(t, tv, key, r.klen);
-          continue;
-        }
-        const greq w = greq_shfl(t, wq, (int)q);
-        if (t.shfl(init, (int)q) == kGAbsent) coop_insert<T, false>(t, tv, cache, key, r.klen, greq_val(g, w), w.vlen);
-        else coop_update<T>(t, tv, cache, key, r.klen, greq_val(g, w), w.vlen);
-      }
-    }
+    int res;
+    if (kind == MT_REQ_INSERT) res = coop_insert<T, false>(t, tv, cache, key, r.klen, greq_val(g, w), w.vlen);
+    else if (kind == MT_REQ_UPDATE) res = coop_update<T>(t, tv, cache, key, r.klen, greq_val(g, w), w.vlen);
+    else res = coop_erase<T>(t, tv, key, r.klen);
+    if (!HEADS && t.leader() && r.d->results) r.d->results[r.i] = res == RES_OK;
   }
   cache.release(t, tv.pool);
 }
@@ -493,25 +451,23 @@ int launch_tile_kernel(mt_masstree* t, void (*fn)(tree_view, grouped_view), cons
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
 }
 
-template <int TF>
-int launch_find_side(mt_masstree* t, const grouped_view& g, cudaStream_t s) {
-  int rc = launch_tile_kernel<TF>(t, group_head_kernel<TF>, g, s);
-  if (rc) return rc;
-  const int grid = std::max(1, std::min<int>(t->sms * 8, (int)((g.m + 255u) / 256u)));
-  group_result_kernel<<<grid, 256, 0, s>>>(g);
+int launch_lanes(mt_masstree* t, void (*fn)(tree_view, grouped_view), const grouped_view& g, cudaStream_t s) {
+  fn<<<host_lane_grid(t, (const void*)fn, g.m), kBlock, 0, s>>>(t->tv, g);
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
 }
 
 template <int TW>
-int launch_singles(mt_masstree* t, const grouped_view& g, cudaStream_t s_ins, cudaStream_t s_ue) {
-  int rc = launch_tile_kernel<TW>(t, group_write_kernel<TW, kGWInsert>, g, s_ins);
-  if (!rc) rc = launch_tile_kernel<TW>(t, group_write_kernel<TW, kGWUpdErase>, g, s_ue);
-  if (!rc) rc = launch_tile_kernel<TW>(t, group_serial_kernel<TW>, g, s_ue);
+int launch_served(mt_masstree* t, const grouped_view& g, cudaStream_t s) {
+  int rc = launch_lanes(t, group_first_kernel, g, s);
+  if (!rc) rc = launch_tile_kernel<TW>(t, group_rest_kernel<TW, false>, g, s);
+  if (!rc) rc = launch_tile_kernel<TW>(t, group_serial_kernel<TW>, g, s);
+  if (rc) return rc;
+  const int grid = std::max(1, std::min<int>(t->sms * 8, (int)((g.m + 255u) / 256u)));
+  group_result_kernel<<<grid, 256, 0, s>>>(g);
+  if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
+  rc = launch_lanes(t, group_final_kernel, g, s);
+  if (!rc) rc = launch_tile_kernel<TW>(t, group_rest_kernel<TW, true>, g, s);
   return rc;
-}
-template <int TW>
-int launch_heads(mt_masstree* t, const grouped_view& g, cudaStream_t s) {
-  return launch_tile_kernel<TW>(t, group_write_kernel<TW, kGWHeads>, g, s);
 }
 
 }  // namespace
@@ -550,8 +506,8 @@ int launch_grouped(mt_masstree* t, const batches_view& b, cudaStream_t s) {
   g.heads = reinterpret_cast<uint32_t*>(carve(M * 4u));
   g.singles = reinterpret_cast<uint32_t*>(carve(M * 4u));
   g.serial = reinterpret_cast<uint32_t*>(carve(M * 4u));
-  g.finds = reinterpret_cast<uint32_t*>(carve(M * 4u));
-  g.singles_ue = reinterpret_cast<uint32_t*>(carve(M * 4u));
+  g.rest = reinterpret_cast<uint32_t*>(carve(M * 4u));
+  g.rest_heads = reinterpret_cast<uint32_t*>(carve(M * 4u));
   void* temp = carve(t->grouped_temp);
   g.counts = b.status + 2;
   if (cudaMemsetAsync(g.counts, 0, 5 * sizeof(uint32_t), s) != cudaSuccess) return MT_ERR_CUDA;
@@ -571,23 +527,7 @@ int launch_grouped(mt_masstree* t, const batches_view& b, cudaStream_t s) {
   group_mark_kernel<<<grid, 256, 0, s>>>(g);
   group_list_kernel<<<grid, 256, 0, s>>>(g);
   if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
-  // Keys touched once (and runs served one by one) on a side stream, beside
-  // the reads, results and final writes of the keys touched more than once:
-  // no key is in both.
-  rc = host_fork(t, s);
-  if (rc) return rc;
-  const bool w16 = t->write_tile_size <= 16;
-  rc = w16 ? launch_singles<16>(t, g, t->side[0], t->side[1]) : launch_singles<32>(t, g, t->side[0], t->side[1]);
-  if (!rc) {
-    switch (t->tile_size) {
-      case 4: rc = launch_find_side<4>(t, g, s); break;
-      case 8: rc = launch_find_side<8>(t, g, s); break;
-      case 16: rc = launch_find_side<16>(t, g, s); break;
-      default: rc = launch_find_side<32>(t, g, s); break;
-    }
-  }
-  if (!rc) rc = w16 ? launch_heads<16>(t, g, s) : launch_heads<32>(t, g, s);
-  return host_join(t, s, rc);
+  return t->write_tile_size <= 16 ? launch_served<16>(t, g, s) : launch_served<32>(t, g, s);
 }
 
 }  // namespace mtb

@@ -231,11 +231,6 @@ struct mt_masstree {
   uint32_t combine_cap = 0;
   uint32_t* defer_mem = nullptr;    // requests the lane kernels hand on: count (one line), then defer_cap entries
   uint32_t defer_cap = 0;
-  // Streams and events of the forked class launches of large mixed batches
-  // (created on first use).
-  cudaStream_t side[2] = {nullptr, nullptr};
-  cudaEvent_t ev_fork = nullptr;
-  cudaEvent_t ev_join[2] = {nullptr, nullptr};
   mt_host_pipe* host_pipe = nullptr;
   void* mem = nullptr;
   mtb::tree_view tv{};
@@ -268,8 +263,6 @@ int host_merge_end(mt_masstree* t, cudaStream_t s, int rc);
 int host_max_blocks_per_sm(const void* fn, int block, size_t smem);
 int host_lane_grid(const mt_masstree* t, const void* fn, uint32_t n);  // blocks for n requests, one per thread
 int host_launch_reclaim(mt_masstree* t, cudaStream_t s);
-int host_fork(mt_masstree* t, cudaStream_t s);
-int host_join(mt_masstree* t, cudaStream_t s, int rc);
 void host_pipe_free(mt_masstree* t);  // mt_host.cu
 // mt_grouped.cu; kGroupedUnavailable: its scratch does not fit, nothing launched.
 constexpr int kGroupedUnavailable = -1001;

@@ -330,58 +330,57 @@ MT_DEV void warp_chains(const pool_view& p, bool want, uint32_t head, const uint
 // spreads few requests over the four groups of warp_chains.
 MT_DEV uint32_t lane_slot(uint32_t lane) { return (lane & 7u) * 4u + (lane >> 3); }
 
-// Finds.  1M finds (half of them misses) on 1M keys of 1-8 slices: 235 us, from
-// 357 us with eight lanes per request (55 warp instructions per find instead
-// of 587).  What bounds it now: a lane's 32-byte loads touch 32 lines per
-// instruction, so the load path moves one sector per cycle (62% busy); the
-// occupancy (4, 6 or 8 blocks per SM) changes nothing.
-template <bool CONC>
-MT_DEV void lane_find(const tree_view& tv, const batch_args& a) {
-  const uint32_t slot = lane_slot(lane_id());
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32u;
-  const uint32_t warps = (gridDim.x * blockDim.x) / 32u;
-  const pool_view& p = tv.pool;
-  const uint32_t nf = a.n_dev ? *a.n_dev : a.n;
-  const uint32_t nb = a.n_back_dev ? *a.n_back_dev : 0u;
-  const uint32_t n = nf + nb;
-  const uint32_t per = max(1u, min(32u, (n + warps - 1u) / warps));
-  uint32_t* values = a.values_out ? a.values_out : a.values;
-#pragma unroll 1
-  for (uint32_t base = warp * per; base < n; base += warps * per) {
-    if (__any_sync(0xFFFFFFFFu, slot == 0u && fatal_error(p))) break;
-    const uint32_t pos = base + slot;
-    const bool valid = slot < per && pos < n;
-    uint32_t i = pos, klen = 0;
-    if (valid) {
-      if (a.index) i = a.index[pos < nf ? pos : a.region - nb + (pos - nf)];
-      klen = a.key_lengths ? a.key_lengths[i] : a.max_key_length;
+// ---- requests --------------------------------------------------------------------
+
+// One request as a lane serves it.  `val`: the value rows of inserts and
+// updates (input) and finds (output; may be null).
+struct lane_request {
+  uint32_t id;  // what the defer list gets
+  uint32_t kind, klen, vlen;
+  const uint32_t* key;
+  uint32_t* val;
+  uint32_t* out_len;  // for sources that do not derive their result addresses from id
+  bool* out_ok;
+};
+enum lane_fetch : uint32_t { LANE_SKIP = 0, LANE_SERVE = 1, LANE_REFUSED = 2 };  // refused: recorded, reported as failed
+
+// Where a kernel's requests come from and its results go to.  fetch is called
+// by single lanes; lane_serve calls found for finds and result for the others.
+struct batch_source {
+  batch_args a;
+  MT_DEV uint32_t size() const { return a.n_dev ? *a.n_dev : a.n; }
+  MT_DEV uint32_t max_value_length() const { return a.max_value_length; }
+  template <int OP>
+  MT_DEV uint32_t fetch(const pool_view& p, uint32_t pos, lane_request& r) const {
+    const uint32_t i = a.index ? a.index[a.first + pos] : a.first + pos;
+    r.id = i;
+    r.kind = MT_REQ_FIND;
+    if (OP == OP_MIXED) r.kind = a.types[i];
+    else if (OP == OP_INSERT || OP == OP_UPSERT) r.kind = MT_REQ_INSERT;
+    else if (OP == OP_UPDATE) r.kind = MT_REQ_UPDATE;
+    else if (OP == OP_ERASE) r.kind = MT_REQ_ERASE;
+    r.klen = a.key_lengths ? a.key_lengths[i] : a.max_key_length;
+    r.vlen = 0;
+    if (r.kind == MT_REQ_INSERT || r.kind == MT_REQ_UPDATE)
+      r.vlen = a.value_lengths_in ? a.value_lengths_in[i] : a.max_value_length;
+    r.key = a.keys + (size_t)i * a.max_key_length;
+    r.val = a.values ? a.values + (size_t)i * a.max_value_length : nullptr;
+    // Lengths beyond the row stride (or unknown kinds) would read outside the
+    // caller's buffers: such requests are skipped and reported.
+    if (r.klen > a.max_key_length || r.vlen > a.max_value_length || r.kind > MT_REQ_UPDATE) {
+      lane_error(p.err, ERR_INVALID_ARG, MT_AT(SRC_LANE));
+      return LANE_REFUSED;
     }
-    const bool bad = valid && klen > a.max_key_length;
-    if (bad) lane_error(p.err, ERR_INVALID_ARG, MT_AT(SRC_LANE));
-    const uint32_t* key = a.keys + (size_t)i * a.max_key_length;
-    uint32_t* out = values ? values + (size_t)i * a.max_value_length : nullptr;
-    lane_place at;
-    bool go = valid && !bad && klen > 0u;
-    lane_locate<CONC>(tv, go, key, klen, at);
-    if (!go) at.found = false;
-    uint32_t vlen = 0;
-    bool chain = at.found && at.state != KS_VALUE;
-    if (chain && !p.valid(at.val)) {
-      lane_error(p.err, ERR_CORRUPT, MT_AT(SRC_LANE));
-      chain = false;
-    }
-    if (at.found && at.state == KS_VALUE) {
-      if (out != nullptr && a.max_value_length > 0u) out[0] = at.val;
-      vlen = 1u;
-    }
-    const uint32_t lk = (chain && at.state == KS_SUFFIX) ? klen - at.layer - 1u : 0u;
-    bool eq = false;
-    uint32_t cv = 0;
-    warp_chains<true>(p, chain, at.val, key + at.layer + 1u, lk, out, a.max_value_length, eq, cv);
-    if (chain && eq) vlen = cv;
-    if (valid && a.value_lengths_out) a.value_lengths_out[i] = vlen;
+    if ((OP == OP_MIXED || OP == OP_UPDATE) && a.leader_of != nullptr && a.leader_of[i] != kInvalid) return LANE_SKIP;
+    return LANE_SERVE;
   }
-}
+  MT_DEV void found(uint32_t, const lane_request& r, bool, uint32_t len) const {
+    if (a.value_lengths_out) a.value_lengths_out[r.id] = len;
+  }
+  MT_DEV void result(uint32_t, const lane_request& r, bool ok) const {
+    if (a.results) a.results[r.id] = ok;
+  }
+};
 
 // ---- writes ------------------------------------------------------------------------
 
@@ -697,8 +696,8 @@ struct defer_list {
   uint32_t* count;
 };
 
-// Serve the requests [a.first, a.first + a.n) (through a.index where given),
-// one per lane and round:
+// Serve the requests of src, one per lane and round (OP_FIND with CONC false:
+// finds that run beside no writer):
 //   1. the lane walks to its border node without locks (lane_locate);
 //   2. eight lanes per request compare suffix chains, copy found values, and
 //      write the chains of inserts and updates (their slabs are taken with one
@@ -717,52 +716,54 @@ struct defer_list {
 // kernel per class and 32 lanes per write (1,505 warp instructions and two
 // fences per insert; now about 500, and the fences serve 32 requests); insert +
 // update + find + erase of 300K keys each on 4M keys 1.58 -> 0.65 ms.
-template <int OP>
-MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_list& dl) {
+// 1M finds (half of them misses) on 1M keys of 1-8 slices: 235 us, from
+// 357 us with eight lanes per request (55 warp instructions per find instead
+// of 587).  What bounds it now: a lane's 32-byte loads touch 32 lines per
+// instruction, so the load path moves one sector per cycle (62% busy); the
+// occupancy (4, 6 or 8 blocks per SM) changes nothing.
+template <int OP, bool CONC, class Src>
+MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl) {
   constexpr uint32_t kAll = 0xFFFFFFFFu;
-  constexpr bool kFinds = OP == OP_MIXED, kInserts = OP == OP_MIXED || OP == OP_INSERT || OP == OP_UPSERT;
+  constexpr bool kFinds = OP == OP_MIXED || OP == OP_FIND;
+  constexpr bool kInserts = OP == OP_MIXED || OP == OP_INSERT || OP == OP_UPSERT;
   constexpr bool kErases = OP == OP_MIXED || OP == OP_ERASE, kUpdates = OP == OP_MIXED || OP == OP_UPDATE;
-  constexpr bool kChains = kInserts || kUpdates;
+  constexpr bool kChains = kInserts || kUpdates, kWrites = kChains || kErases;
   const uint32_t slot = lane_slot(lane_id());
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32u;
   const uint32_t warps = (gridDim.x * blockDim.x) / 32u;
   const pool_view& p = tv.pool;
-  const uint32_t per = max(1u, min(32u, (a.n + warps - 1u) / warps));
+  const uint32_t n = src.size(), maxV = src.max_value_length();
+  const uint32_t per = max(1u, min(32u, (n + warps - 1u) / warps));
   uint32_t shard = (warp * 0x9E3779B1u) % p.num_shards;
 #pragma unroll 1
-  for (uint32_t base = warp * per; base < a.n; base += warps * per) {
+  for (uint32_t base = warp * per; base < n; base += warps * per) {
     if (__any_sync(kAll, slot == 0u && fatal_error(p))) break;
     const uint32_t pos = base + slot;
-    const bool valid = slot < per && pos < a.n;
-    uint32_t i = 0, kind = 0, klen = 0, vlen = 0;
-    if (valid) {
-      i = a.index ? a.index[a.first + pos] : a.first + pos;
-      kind = OP == OP_MIXED ? (uint32_t)a.types[i]
-                            : (uint32_t)(kInserts ? MT_REQ_INSERT : (kUpdates ? MT_REQ_UPDATE : MT_REQ_ERASE));
-      klen = a.key_lengths ? a.key_lengths[i] : a.max_key_length;
-      if (kChains && (kind == MT_REQ_INSERT || kind == MT_REQ_UPDATE))
-        vlen = a.value_lengths_in ? a.value_lengths_in[i] : a.max_value_length;
-    }
-    const bool bad = valid && (klen > a.max_key_length || vlen > a.max_value_length || kind > MT_REQ_UPDATE);
-    if (bad) lane_error(p.err, ERR_INVALID_ARG, MT_AT(SRC_LANE));
-    bool combined = false;
-    if (kUpdates && valid && a.leader_of != nullptr) combined = a.leader_of[i] != kInvalid;
-    const bool act = valid && !bad && !combined;
-    const uint32_t* key = a.keys + (size_t)i * a.max_key_length;
-    uint32_t* val = a.values + (size_t)i * a.max_value_length;
-    const bool find = kFinds && act && kind == MT_REQ_FIND;
-    const bool insert = kInserts && act && kind == MT_REQ_INSERT;
-    const bool update = kUpdates && act && kind == MT_REQ_UPDATE;
-    const bool erase = kErases && act && kind == MT_REQ_ERASE;
+    lane_request r;
+    r.id = r.kind = r.klen = r.vlen = 0;
+    r.key = nullptr;
+    r.val = nullptr;
+    r.out_len = nullptr;
+    r.out_ok = nullptr;
+    uint32_t have = LANE_SKIP;
+    if (slot < per && pos < n) have = src.template fetch<OP>(p, pos, r);
+    const bool act = have == LANE_SERVE;
+    const uint32_t klen = r.klen, vlen = r.vlen;
+    const uint32_t* key = r.key;
+    uint32_t* val = r.val;
+    const bool find = kFinds && act && r.kind == MT_REQ_FIND;
+    const bool insert = kInserts && act && r.kind == MT_REQ_INSERT;
+    const bool update = kUpdates && act && r.kind == MT_REQ_UPDATE;
+    const bool erase = kErases && act && r.kind == MT_REQ_ERASE;
     if (kChains && (insert || update)) asm volatile("prefetch.global.L2 [%0];" ::"l"(val));
-    bool defer = (insert || update) && (klen == 0u || klen > kMaxLen16 || vlen > kMaxLen16);
+    bool defer = kChains && (insert || update) && (klen == 0u || klen > kMaxLen16 || vlen > kMaxLen16);
     bool go = act && !defer && klen > 0u;
 
     // 1. To the border node.
     lane_place at;
     at.idx = 0;
     at.full = false;
-    lane_locate<true>(tv, go, key, klen, at);
+    lane_locate<CONC>(tv, go, key, klen, at);
     bool chain = go && at.found && (at.state == KS_SUFFIX || (find && at.state == KS_LONGVAL));
     if (chain && !p.valid(at.val)) {
       lane_error(p.err, ERR_CORRUPT, MT_AT(SRC_LANE));
@@ -775,11 +776,11 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
     if (chain) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.addr(at.val)));
     bool eq = false;
     uint32_t cv = 0, res = 0, found_len = 0;
-    warp_chains<kFinds>(p, chain, at.val, key + at.layer + 1u, rest, find ? val : nullptr, a.max_value_length, eq, cv);
+    warp_chains<kFinds>(p, chain, at.val, key + at.layer + 1u, rest, find ? val : nullptr, maxV, eq, cv);
     const bool present = go && at.found && (at.state != KS_SUFFIX || eq);
     if (find && present) {
       if (at.state == KS_VALUE) {
-        val[0] = at.val;
+        if (val != nullptr && maxV > 0u) val[0] = at.val;
         found_len = 1u;
       } else {
         found_len = cv;
@@ -823,7 +824,7 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
     const uint32_t slice = klen > 0u && act ? key[at.layer] : 0u;
     uint32_t idx = at.idx, tries = 0, old_chain = kInvalid;
 #pragma unroll 1
-    while (__any_sync(kAll, job != JOB_NONE)) {
+    while (kWrites && __any_sync(kAll, job != JOB_NONE)) {
       uint32_t w[32];
       bool won = false, split = false, parent_ok = false;
       uint32_t e = 0, pslot = 0, pmeta = 0;
@@ -958,23 +959,22 @@ MT_DEV void lane_serve(const tree_view& tv, const batch_args& a, const defer_lis
     }
     // Chains replaced or erased, and slabs taken in vain.
     if (kChains && (ns & KS_SLAB) && nv != kInvalid) old_chain = nv;
-    if (old_chain != kInvalid) lane_retire_chain(p, old_chain);
+    if (kWrites && old_chain != kInvalid) lane_retire_chain(p, old_chain);
     if (kInserts && spare != kInvalid) retire_slab(p, spare);
 
     // 4. Results, and the requests left to the tile kernel.
-    const uint32_t dm = __ballot_sync(kAll, defer);
-    if (dm) {
-      uint32_t at0 = 0;
-      if (lane_id() == 0u) at0 = atomicAdd(dl.count, (uint32_t)__popc(dm));
-      at0 = __shfl_sync(kAll, at0, 0);
-      if (defer) dl.list[at0 + __popc(dm & ((1u << lane_id()) - 1u))] = i;
-    }
-    if (valid && !combined && !defer) {
-      if (kFinds && kind == MT_REQ_FIND) {
-        if (a.value_lengths_out) a.value_lengths_out[i] = found_len;
-      } else if (a.results) {
-        a.results[i] = res != 0u;
+    if (kWrites) {
+      const uint32_t dm = __ballot_sync(kAll, defer);
+      if (dm) {
+        uint32_t at0 = 0;
+        if (lane_id() == 0u) at0 = atomicAdd(dl.count, (uint32_t)__popc(dm));
+        at0 = __shfl_sync(kAll, at0, 0);
+        if (defer) dl.list[at0 + __popc(dm & ((1u << lane_id()) - 1u))] = r.id;
       }
+    }
+    if (have != LANE_SKIP && !defer) {
+      if (kFinds && r.kind == MT_REQ_FIND) src.found(pos, r, present, found_len);
+      else src.result(pos, r, res != 0u);
     }
   }
 }
