@@ -97,16 +97,34 @@ __global__ void bulk_classify_kernel(bulk_view b) {
   if (threadIdx.x == 0) b.block_entries[blockIdx.x] = c;
 }
 
-// Exclusive sums of the per-block counts (one thread); ctl[3] = total.
-__global__ void bulk_block_scan_kernel(bulk_view b, uint32_t nblocks) {
-  if (threadIdx.x != 0) return;
-  uint32_t run = 0;
-  for (uint32_t k = 0; k < nblocks; ++k) {
-    const uint32_t c = b.block_entries[k];
-    b.block_entries[k] = run;
-    run += c;
+// Exclusive sums of the per-block counts (one block of 1,024 threads);
+// ctl[3] = total.  (One thread summing the 4,096 counts of 1M keys waited for
+// each load in turn.)
+__global__ void __launch_bounds__(1024) bulk_block_scan_kernel(bulk_view b, uint32_t nblocks) {
+  __shared__ uint32_t warp_sum[32];
+  __shared__ uint32_t carry;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) carry = 0u;
+  __syncthreads();
+  for (uint32_t base = 0; base < nblocks; base += 1024u) {
+    const uint32_t k = base + threadIdx.x;
+    const uint32_t c = k < nblocks ? b.block_entries[k] : 0u;
+    uint32_t incl = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= (uint32_t)d) incl += up;
+    }
+    if (lane == 31u) warp_sum[warp] = incl;
+    __syncthreads();
+    uint32_t below = carry;
+    for (uint32_t w = 0; w < warp; ++w) below += warp_sum[w];
+    if (k < nblocks) b.block_entries[k] = below + incl - c;
+    __syncthreads();
+    if (threadIdx.x == 1023u) carry = below + incl;
+    __syncthreads();
   }
-  b.ctl[3] = run;
+  if (threadIdx.x == 0) b.ctl[3] = carry;
 }
 
 // Pass 2: the entries, in key order, to the entry arrays.
@@ -148,7 +166,12 @@ __global__ void __launch_bounds__(kBlock, MT_MIN_BLOCKS_PER_SM) bulk_entry_kerne
   cache.init(tv.pool, tile_id);
   const pool_view& p = tv.pool;
   nu = min(nu, b.ctl[3]);  // entries found by the compaction (nu: capacity)
-  for (uint32_t u = tile_id; u < nu; u += num_tiles) {
+  // A tile takes up to 32 entries in key order at a time, so that their chains
+  // come from one refill of its slab cache and lie side by side: a scan reads
+  // them one after the other.
+  const uint32_t run = max(1u, min(32u, nu / num_tiles));
+  for (uint32_t base = tile_id * run; base < nu; base += num_tiles * run)
+  for (uint32_t u = base; u < min(base + run, nu); ++u) {
     if (t.shfl((uint32_t)(t.leader() && fatal_error(p)), 0)) break;
     const uint32_t i = b.e_src[u];
     if (i == kInvalid) {
@@ -200,10 +223,13 @@ __global__ void __launch_bounds__(kBlock, MT_MIN_BLOCKS_PER_SM) bulk_alloc_kerne
   const uint32_t tile_id = (blockIdx.x * blockDim.x + threadIdx.x) / 32u;
   const uint32_t num_tiles = (gridDim.x * blockDim.x) / 32u;
   cache.init(tv.pool, tile_id);
-  for (uint32_t k = tile_id; k < count; k += num_tiles) {
-    const uint32_t s = count == 1u ? root : cache.allocate(t, tv.pool);
-    if (t.leader()) ids[k] = s;
-  }
+  // Nodes in key order side by side, as the chains (bulk_entry_kernel).
+  const uint32_t run = max(1u, min(32u, count / num_tiles));
+  for (uint32_t base = tile_id * run; base < count; base += num_tiles * run)
+    for (uint32_t k = base; k < min(base + run, count); ++k) {
+      const uint32_t s = count == 1u ? root : cache.allocate(t, tv.pool);
+      if (t.leader()) ids[k] = s;
+    }
   cache.release(t, tv.pool);
 }
 
@@ -338,7 +364,7 @@ int host_bulk_insert(mt_masstree* t, const batch_args& a, bool upsert, cudaStrea
                                             kBulkSortBits, s));
   if (!rc) {
     bulk_classify_kernel<<<cblocks, 256, 0, s>>>(b);
-    bulk_block_scan_kernel<<<1, 32, 0, s>>>(b, cblocks);
+    bulk_block_scan_kernel<<<1, 1024, 0, s>>>(b, cblocks);
     bulk_compact_kernel<<<cblocks, 256, 0, s>>>(b);
     rc = cu(cudaGetLastError());
   }
@@ -380,7 +406,8 @@ int host_bulk_insert(mt_masstree* t, const batch_args& a, bool upsert, cudaStrea
     }
   }
   if (!rc && h[2] > 0u) {
-    // The rest through the ordinary insert kernel.
+    // The rest through the ordinary insert kernel (its tile form: in a tree
+    // this young, lanes would hand most of them on).
     batch_args r = a;
     r.index = b.rest;
     r.n = h[2];
