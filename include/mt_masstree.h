@@ -54,7 +54,7 @@ enum { MT_REQ_INSERT = 0, MT_REQ_ERASE = 1, MT_REQ_FIND = 2, MT_REQ_UPDATE = 3 }
                                        every request class (accepted by mixed_batch, which
                                        serves its requests without classes) */
 #define MT_FLAG_PERSISTENT 32u      /* mixed_batches: one cooperative persistent launch for all
-                                       sub-batches instead of three class kernels per sub-batch */
+                                       sub-batches instead of a kernel pair per sub-batch */
 #define MT_FLAG_MERGE 64u           /* erase, mixed_batch: after the call's erases, fold nodes
                                        left with 4 entries or fewer into a neighbour under the same
                                        parent, border nodes and then their sparse ancestors, and
@@ -105,29 +105,34 @@ typedef struct mt_stats_t {
 
 /* Construction.  Replaces gpu_masstree(allocator(pool_ratio), reclaimer())
  * (reference gpu_masstree.hpp:67-72, simple_slab_alloc.hpp:56-69): the slab
- * pool takes pool_ratio of the currently free device memory.  tile_size is the
- * number of lanes serving one request (4, 8, 16 or 32). */
+ * pool takes pool_ratio of the currently free device memory (a little is
+ * allocated beside it: counters and a list of at most 1/256 of the pool).
+ * tile_size: see mt_set_tile_size. */
 int mt_create(mt_masstree** out, float pool_ratio, uint32_t tile_size);
 /* Same, with the pool size given in bytes. */
 int mt_create_bytes(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size);
 /* Reference ~gpu_masstree / ~simple_slab_allocator (gpu_masstree.hpp:80-82). */
 int mt_destroy(mt_masstree* tree);
 
-/* Launch shape: lanes per request (4/8/16/32) and resident blocks per SM
- * (0 = as many as fit).  New in this library. */
+/* Launch shape: lanes per request (4/8/16/32) of the kernels that serve a
+ * request with a tile of lanes (serving loop, MT_FLAG_PERSISTENT,
+ * MT_FLAG_SINGLE_PASS, mt_mixed_batch_noalloc's writes, and the requests that
+ * the one-request-per-lane kernels of the batch calls hand on), and resident
+ * blocks per SM (0 = as many as fit).  The batch calls themselves serve one
+ * request per lane, scans 16 lanes per query, whatever the width.  New in this
+ * library. */
 int mt_set_tile_size(mt_masstree* tree, uint32_t tile_size);
 /* Lanes per request for inserts, updates and erases only (mt_set_tile_size
  * sets both widths). */
 int mt_set_write_tile_size(mt_masstree* tree, uint32_t tile_size);
 int mt_set_blocks_per_sm(mt_masstree* tree, uint32_t blocks_per_sm);
 /* Lanes per update or erase request of mixed batches (4/8/16/32; 0 = the
- * write width, the default).  Under skewed key choice most of them miss (the
- * key was erased) and end in a lock-free check, which narrow tiles serve many
- * at a time.  New in this library. */
+ * write width, the default).  Accepted and kept; mixed batches serve one
+ * request per lane.  New in this library. */
 int mt_set_upderase_tile_size(mt_masstree* tree, uint32_t tile_size);
-/* Lanes per scan query (4/8/16/32; 0 = the find width, the default).  Scans
- * read many independent suffix lines per query and run fastest with narrow
- * tiles (more queries in flight).  New in this library. */
+/* Lanes per scan query (4/8/16/32; 0 = the find width, the default).  Accepted
+ * and kept; scans use 16 lanes, one per entry of the border node at hand.  New
+ * in this library. */
 int mt_set_scan_tile_size(mt_masstree* tree, uint32_t tile_size);
 
 /* Bound of every node-lock wait: lock attempts (each followed by a backoff of
@@ -219,17 +224,17 @@ int mt_batches_reserve(mt_masstree* tree, uint32_t max_subbatches, uint64_t max_
 
 /* Serve num_subbatches mixed batches in order, with the results of one
  * mt_mixed_batch call per sub-batch: sub-batch k+1 sees every effect of
- * sub-batch k.  One partition pass files every request of every sub-batch
- * under its class; then, by default, each sub-batch runs its three class
- * kernels side by side on forked streams (3 launches per sub-batch), or, with
- * MT_FLAG_PERSISTENT, one cooperative persistent launch serves all
+ * sub-batch k.  By default each sub-batch is one kernel, one request per lane,
+ * and a second one for the few requests that the first hands on; with
+ * MT_FLAG_PERSISTENT a partition pass files every request of every sub-batch
+ * under its class and one cooperative persistent launch serves all
  * sub-batches with a grid barrier between them.  `subbatches` is a DEVICE
  * array of descriptors; nothing is read back to the host and the number of
  * launches depends only on num_subbatches, so the call can be captured in a
  * CUDA graph and replayed after the descriptors' contents change.  Needs
  * mt_batches_reserve; flags may hold MT_FLAG_BUCKET_KEYS and
- * MT_FLAG_PERSISTENT.  Find tile width: mt_set_tile_size (4/8/16/32); write
- * tile width: mt_set_write_tile_size (16 or 32).  With MT_FLAG_GROUP_BY_KEY
+ * MT_FLAG_PERSISTENT (whose find tile width is mt_set_tile_size's, 4/8/16/32,
+ * and write tile width mt_set_write_tile_size's, 16 or 32).  With MT_FLAG_GROUP_BY_KEY
  * all sub-batches are served at once: the requests are sorted by a hash of
  * their key, each key's requests resolved in sub-batch order (and, inside a
  * sub-batch, in buffer order) by a segmented scan, the tree read once and

@@ -31,15 +31,27 @@ namespace cg = cooperative_groups;
 namespace mtb {
 
 __global__ void batches_prepare_kernel(batches_view b, pool_view p) {
-  if (threadIdx.x == 0) {
+  // Exclusive sums of the sizes by the first warp, 32 sub-batches a round (a
+  // single thread waited for each descriptor in turn).
+  if (threadIdx.x < 32u) {
     uint64_t acc = 0;
-    for (uint32_t s = 0; s < b.nsub; ++s) {
-      b.offsets[s] = (uint32_t)min(acc, (uint64_t)0xFFFFFFFFu);
-      acc += b.sub[s].num_requests;
+    for (uint32_t base = 0; base < b.nsub; base += 32u) {
+      const uint32_t s = base + threadIdx.x;
+      const uint64_t c = s < b.nsub ? b.sub[s].num_requests : 0u;
+      uint64_t incl = c;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t up = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (threadIdx.x >= (uint32_t)d) incl += up;
+      }
+      if (s < b.nsub) b.offsets[s] = (uint32_t)min(acc + incl - c, (uint64_t)0xFFFFFFFFu);
+      acc += __shfl_sync(0xFFFFFFFFu, incl, 31);
     }
-    b.offsets[b.nsub] = (uint32_t)min(acc, (uint64_t)0xFFFFFFFFu);
-    b.status[0] = acc > b.max_total ? 1u : 0u;
-    if (acc > b.max_total) record_error(p, ERR_INVALID_ARG);
+    if (threadIdx.x == 0u) {
+      b.offsets[b.nsub] = (uint32_t)min(acc, (uint64_t)0xFFFFFFFFu);
+      b.status[0] = acc > b.max_total ? 1u : 0u;
+      if (acc > b.max_total) record_error(p, ERR_INVALID_ARG);
+    }
   }
   for (uint32_t i = threadIdx.x; i < b.nsub * kCountStride; i += blockDim.x) b.counts[i] = 0u;
 }

@@ -62,6 +62,13 @@ __global__ void partition_kernel(const uint8_t* types, uint32_t n, uint32_t* fin
 // by a hash of the key; the first request of a key owns its slot, the others
 // compare keys and record that request in leader_of.  The batch kernel skips
 // them, and combine_results_kernel copies the leader's result.
+//
+// The table is never cleared between calls: an entry is (epoch << 32 | request),
+// and the epoch, a device word that every call's reclaim pass moves (so that
+// replayed graphs move it too), makes the entries of earlier calls free.  A block
+// first gathers its updates, then works on them with every lane: in a mixed
+// batch with a tenth of updates a warp's three updates otherwise waited for
+// their key rows while the other lanes idled.
 MT_DEV uint64_t key_hash(const uint32_t* k, uint32_t klen) {
   uint64_t h = 0x9E3779B97F4A7C15ull ^ klen;
   for (uint32_t q = 0; q < klen; ++q) {
@@ -72,42 +79,62 @@ MT_DEV uint64_t key_hash(const uint32_t* k, uint32_t klen) {
   return h ^ (h >> 29);
 }
 
-MT_DEV uint32_t class_request(const batch_args& a, uint32_t pos, uint32_t nf, uint32_t nb) {
-  return a.index ? a.index[pos < nf ? pos : a.region - nb + (pos - nf)] : pos;
-}
-
-__global__ void combine_kernel(batch_args a, uint32_t* table, uint32_t mask, uint32_t* leader_of) {
-  const uint32_t nf = a.n_dev ? *a.n_dev : a.n;
-  const uint32_t nb = a.n_back_dev ? *a.n_back_dev : 0u;
-  for (uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x; pos < nf + nb; pos += gridDim.x * blockDim.x) {
-    const uint32_t i = class_request(a, pos, nf, nb);
-    if (a.types && a.types[i] != MT_REQ_UPDATE) continue;
-    const uint32_t klen = a.key_lengths ? a.key_lengths[i] : a.max_key_length;
-    const uint32_t vlen = a.value_lengths_in ? a.value_lengths_in[i] : a.max_value_length;
-    if (klen == 0u || klen > a.max_key_length || vlen > a.max_value_length) continue;  // reported when served
-    const uint32_t* k = a.keys + (size_t)i * a.max_key_length;
-    uint32_t slot = (uint32_t)key_hash(k, klen) & mask;
-    for (uint32_t probe = 0; probe <= mask; ++probe) {
-      const uint32_t j = atomicCAS(table + slot, kInvalid, i);
-      if (j == kInvalid) break;  // i leads its key
-      const uint32_t jl = a.key_lengths ? a.key_lengths[j] : a.max_key_length;
-      bool same = jl == klen;
-      const uint32_t* kj = a.keys + (size_t)j * a.max_key_length;
-      for (uint32_t q = 0; same && q < klen; ++q) same = kj[q] == k[q];
-      if (same) {
-        leader_of[i] = j;
-        break;
+constexpr uint32_t kCombineChunk = 1024;  // requests that a block looks at together
+__global__ void __launch_bounds__(256) combine_kernel(batch_args a, unsigned long long* table, uint32_t mask,
+                                                      uint32_t* leader_of, const uint32_t* epoch_word) {
+  __shared__ uint32_t list[kCombineChunk];
+  __shared__ uint32_t count;
+  const unsigned long long epoch = *epoch_word;
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t base = blockIdx.x * kCombineChunk; base < a.n; base += gridDim.x * kCombineChunk) {
+    if (threadIdx.x == 0) count = 0u;
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < kCombineChunk; q += 256u) {
+      const uint32_t i = base + q;
+      bool update = false;
+      if (i < a.n) {
+        leader_of[i] = kInvalid;
+        update = a.types == nullptr || a.types[i] == MT_REQ_UPDATE;
       }
-      slot = (slot + 1u) & mask;
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, update);
+      uint32_t at = 0;
+      if (lane == 0 && m) at = atomicAdd(&count, (uint32_t)__popc(m));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0);
+      if (update) list[at + __popc(m & ((1u << lane) - 1u))] = i;
     }
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < count; q += 256u) {
+      const uint32_t i = list[q];
+      const uint32_t klen = a.key_lengths ? a.key_lengths[i] : a.max_key_length;
+      const uint32_t vlen = a.value_lengths_in ? a.value_lengths_in[i] : a.max_value_length;
+      if (klen == 0u || klen > a.max_key_length || vlen > a.max_value_length) continue;  // reported when served
+      const uint32_t* k = a.keys + (size_t)i * a.max_key_length;
+      uint32_t slot = (uint32_t)key_hash(k, klen) & mask;
+      for (uint32_t probe = 0; probe <= mask; ++probe) {
+        unsigned long long cur = *(volatile unsigned long long*)(table + slot);
+        if ((cur >> 32) != epoch) {
+          const unsigned long long old = atomicCAS(table + slot, cur, (epoch << 32) | i);
+          if (old == cur) break;  // i leads its key
+          cur = old;              // another request of this call took the slot
+        }
+        const uint32_t j = (uint32_t)cur;
+        const uint32_t jl = a.key_lengths ? a.key_lengths[j] : a.max_key_length;
+        bool same = jl == klen;
+        const uint32_t* kj = a.keys + (size_t)j * a.max_key_length;
+        for (uint32_t w = 0; same && w < klen; ++w) same = kj[w] == k[w];
+        if (same) {
+          leader_of[i] = j;
+          break;
+        }
+        slot = (slot + 1u) & mask;
+      }
+    }
+    __syncthreads();
   }
 }
 
 __global__ void combine_results_kernel(batch_args a, const uint32_t* leader_of) {
-  const uint32_t nf = a.n_dev ? *a.n_dev : a.n;
-  const uint32_t nb = a.n_back_dev ? *a.n_back_dev : 0u;
-  for (uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x; pos < nf + nb; pos += gridDim.x * blockDim.x) {
-    const uint32_t i = class_request(a, pos, nf, nb);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
     const uint32_t j = leader_of[i];
     if (j != kInvalid) a.results[i] = a.results[j];
   }
@@ -228,10 +255,13 @@ __global__ void line_atomicity_kernel(uint32_t* lines, uint32_t nlines, uint32_t
   }
 }
 
-// Return slabs retired by earlier launches to their shard's free stack, and
-// start the call's defer list (may be null) empty.
-__global__ void reclaim_kernel(pool_view p, uint32_t* defer_count) {
-  if (blockIdx.x == 0 && threadIdx.x == 0 && defer_count != nullptr) *defer_count = 0u;
+// Return slabs retired by earlier launches to their shard's free stack; start
+// the call's defer list empty (call[0]) and its epoch (call[1]).
+__global__ void reclaim_kernel(pool_view p, uint32_t* call) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    call[0] = 0u;
+    call[1] += 1u;
+  }
   for (uint32_t s = blockIdx.x; s < p.num_shards; s += gridDim.x) {
     __shared__ int top, n;
     if (threadIdx.x == 0) {
@@ -344,10 +374,10 @@ int launch_batch_tile(mt_masstree* t, uint32_t tile, const batch_args& a, cudaSt
 // Writes and mixed batches: the lane kernel, then a tile kernel for the
 // requests it hands on (few: splits of roots and full parents, new layers,
 // nodes under contention), in pieces that fit the defer list.
+// The reclaim pass is the caller's.
 template <int OP>
 int launch_lane(mt_masstree* t, batch_args a, uint32_t tile, cudaStream_t s) {
-  if (a.n == 0) return MT_OK;
-  int rc = launch_reclaim(t, s);
+  int rc = MT_OK;
   const defer_list dl{t->defer_mem + 32, t->defer_mem};
   const uint32_t n = a.n;
   for (uint32_t first = 0; !rc && first < n; first += a.n) {
@@ -364,8 +394,10 @@ int launch_lane(mt_masstree* t, batch_args a, uint32_t tile, cudaStream_t s) {
   return rc;
 }
 template <int OP>
-int launch_lane(mt_masstree* t, const batch_args& a, cudaStream_t s) {
-  return launch_lane<OP>(t, a, t->write_tile_size, s);
+int launch_writes(mt_masstree* t, const batch_args& a, cudaStream_t s) {
+  if (a.n == 0) return MT_OK;
+  const int rc = launch_reclaim(t, s);
+  return rc ? rc : launch_lane<OP>(t, a, t->write_tile_size, s);
 }
 
 // Finds take no slabs, so no reclaim pass precedes them.  a.n: the number of
@@ -393,29 +425,29 @@ uint32_t combine_slots(uint32_t n) {
 }
 
 // Combining scratch for n requests (grown on demand, kept): the table of
-// combine_slots(n) words, then leader_of (n words).
+// combine_slots(n) entries, then leader_of (n words).
 int ensure_combine_scratch(mt_masstree* t, uint32_t n, cudaStream_t s) {
   if (n <= t->combine_cap) return MT_OK;
   if (cudaStreamSynchronize(s) != cudaSuccess) return MT_ERR_CUDA;
   if (t->combine_mem) cudaFree(t->combine_mem);
   t->combine_mem = nullptr;
   t->combine_cap = 0;
-  if (cudaMalloc(&t->combine_mem, ((size_t)n + combine_slots(n)) * sizeof(uint32_t)) != cudaSuccess) return MT_ERR_OOM;
+  const size_t table = (size_t)combine_slots(n) * sizeof(unsigned long long);
+  if (cudaMalloc(&t->combine_mem, table + (size_t)n * sizeof(uint32_t)) != cudaSuccess) return MT_ERR_OOM;
   t->combine_cap = n;
-  return MT_OK;
+  // Epoch 0, before every call's.
+  return cuda_status(cudaMemsetAsync(t->combine_mem, 0, table, s));
 }
 
-// Combine the updates among the requests of `a` on stream s and set
-// a.leader_of for the kernels that follow.
+// Combine the updates among the requests of `a` on stream s (after the call's
+// reclaim pass) and set a.leader_of for the kernels that follow.
 int launch_combine(mt_masstree* t, batch_args& a, cudaStream_t s) {
-  int rc = ensure_combine_scratch(t, a.n, s);
-  if (rc) return rc;
-  const uint32_t slots = combine_slots(a.n);
-  uint32_t* table = t->combine_mem;
-  uint32_t* leader_of = table + slots;
-  if (cudaMemsetAsync(table, 0xFF, ((size_t)slots + a.n) * sizeof(uint32_t), s) != cudaSuccess) return MT_ERR_CUDA;
-  combine_kernel<<<std::max(1, std::min(t->sms * 8, (int)((a.n + 255) / 256))), 256, 0, s>>>(a, table, slots - 1u,
-                                                                                             leader_of);
+  const uint32_t slots = combine_slots(t->combine_cap);
+  auto* table = reinterpret_cast<unsigned long long*>(t->combine_mem);
+  uint32_t* leader_of = reinterpret_cast<uint32_t*>(table + slots);
+  const uint32_t mask = combine_slots(a.n) - 1u;  // a small call stays within a small part of the table
+  const int grid = std::max(1, std::min<int>(t->sms * 8, (int)((a.n + kCombineChunk - 1u) / kCombineChunk)));
+  combine_kernel<<<grid, 256, 0, s>>>(a, table, mask, leader_of, t->defer_mem + 1);
   if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
   a.leader_of = leader_of;
   return MT_OK;
@@ -431,7 +463,9 @@ int launch_combine_results(mt_masstree* t, const batch_args& a, uint32_t n, cuda
 // serves its own, whatever its kind (a walk is the same for all kinds).
 int launch_mixed(mt_masstree* t, batch_args a, cudaStream_t s) {
   if (a.n == 0) return MT_OK;
-  int rc = launch_combine(t, a, s);
+  int rc = ensure_combine_scratch(t, a.n, s);
+  if (!rc) rc = launch_reclaim(t, s);
+  if (!rc) rc = launch_combine(t, a, s);
   if (!rc) rc = launch_lane<OP_MIXED>(t, a, t->write_tile_size <= 16 ? 16u : 32u, s);
   if (!rc) rc = launch_combine_results(t, a, a.n, s);
   return rc;
@@ -497,7 +531,7 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
   p.num_shards = kShards;
   p.shard_slabs = shard_slabs;
   p.lock_spins = kLockSpins;
-  cudaError_t e = cudaMemset(p.ctr, 0, ctr_bytes + err_bytes);
+  cudaError_t e = cudaMemset(p.ctr, 0, ctr_bytes + err_bytes + 128);  // and the call words in front of the defer list
   // Root of trie layer 0 = slab 0 (shard 0's bump pointer starts past it).
   uint32_t root_img[32] = {0};
   root_img[WORD_HIGH] = 0xFFFFFFFFu;
@@ -523,7 +557,10 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
 
 namespace mtb {
 int host_launch_insert(mt_masstree* t, const batch_args& a, bool upsert, cudaStream_t s) {
-  return upsert ? launch_lane<OP_UPSERT>(t, a, s) : launch_lane<OP_INSERT>(t, a, s);
+  const int rc = launch_reclaim(t, s);
+  if (rc) return rc;
+  return upsert ? launch_batch_tile<OP_UPSERT, true>(t, t->write_tile_size, a, s)
+                : launch_batch_tile<OP_INSERT, true>(t, t->write_tile_size, a, s);
 }
 }  // namespace mtb
 
@@ -647,7 +684,7 @@ int mt_insert(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_
     }
   }
   if (n) t->maybe_empty = false;
-  return upsert ? launch_lane<OP_UPSERT>(t, a, s) : launch_lane<OP_INSERT>(t, a, s);
+  return upsert ? launch_writes<OP_UPSERT>(t, a, s) : launch_writes<OP_INSERT>(t, a, s);
 }
 
 int mt_update(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_t* klens, const uint32_t* values,
@@ -658,9 +695,11 @@ int mt_update(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_
   a.keys = keys; a.key_lengths = klens; a.values = const_cast<uint32_t*>(values); a.value_lengths_in = vlens;
   a.results = results; a.max_key_length = maxK; a.max_value_length = maxV; a.n = n;
   const cudaStream_t s = (cudaStream_t)stream;
-  if (n < 2) return launch_lane<OP_UPDATE>(t, a, s);
-  int rc = launch_combine(t, a, s);
-  if (!rc) rc = launch_lane<OP_UPDATE>(t, a, s);
+  if (n < 2) return launch_writes<OP_UPDATE>(t, a, s);
+  int rc = ensure_combine_scratch(t, n, s);
+  if (!rc) rc = launch_reclaim(t, s);
+  if (!rc) rc = launch_combine(t, a, s);
+  if (!rc) rc = launch_lane<OP_UPDATE>(t, a, t->write_tile_size, s);
   if (!rc) rc = launch_combine_results(t, a, n, s);
   return rc;
 }
@@ -671,10 +710,10 @@ int mt_erase(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_t
   batch_args a{};
   a.keys = keys; a.key_lengths = klens; a.results = results; a.max_key_length = maxK; a.n = n;
   const cudaStream_t s = (cudaStream_t)stream;
-  if (!(flags & (MT_FLAG_MERGE | MT_FLAG_REMOVE_EMPTY_LAYERS))) return launch_lane<OP_ERASE>(t, a, s);
+  if (!(flags & (MT_FLAG_MERGE | MT_FLAG_REMOVE_EMPTY_LAYERS))) return launch_writes<OP_ERASE>(t, a, s);
   const int rc = host_merge_begin(t, s, flags);
   if (rc) return rc;
-  return host_merge_end(t, s, launch_lane<OP_ERASE>(t, a, s));
+  return host_merge_end(t, s, launch_writes<OP_ERASE>(t, a, s));
 }
 
 int mt_mixed_batch(mt_masstree* t, const uint8_t* types, const uint32_t* keys, uint32_t maxK,
