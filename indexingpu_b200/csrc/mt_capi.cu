@@ -1,13 +1,15 @@
 // Batch kernels and the C ABI of libmt_b200.so.
 //
-// Every host call is one stream-ordered launch of a persistent grid-stride
-// kernel (the reference's batch_kernel, include/kernels.hpp:31-103), preceded by
-// the reclaim pass that returns slabs retired by earlier calls.  Differences:
+// A host call is a short, fixed sequence of stream-ordered launches: the reclaim
+// pass that returns slabs retired by earlier calls (not for finds), a
+// grid-stride kernel that serves one request per lane (mt_lane.cuh), and a tile
+// kernel for the requests that it hands on (the reference launches one tile
+// kernel, include/kernels.hpp:31-103).  Differences:
 //   * the launch shape (blocks per SM from the occupancy API, SM count) is
 //     computed once per kernel and cached, not on every call (the reference
 //     queries it per call, kernels.hpp:91-99);
-//   * a tile serves T requests per round, loading their metadata coalesced
-//     (one request per lane) and writing results coalesced;
+//   * a warp serves 32 requests per round, one per lane (a tile T of them),
+//     loading their metadata and writing their results coalesced;
 //   * there is no block-wide barrier per round: reclamation is launch-granular
 //     (see mt_pool.cuh).
 #include <cuda_runtime.h>
@@ -156,8 +158,8 @@ __global__ void __launch_bounds__(kBlock, MT_LANE_FIND_BLOCKS) find_kernel(tree_
   lane_serve<OP_FIND, CONC>(tv, batch_source{a}, defer_list{nullptr, nullptr});
 }
 
-// Inserts, updates, erases and mixed batches, one request per lane.  4M-key
-// and 16M-key trees: see lane_serve.
+// Inserts, updates, erases and mixed batches, one request per lane (what bounds
+// them and what they measured: lane_serve).
 template <int OP>
 __global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) lane_kernel(tree_view tv, batch_args a, defer_list dl) {
   lane_serve<OP, true>(tv, batch_source{a}, dl);

@@ -712,15 +712,14 @@ struct defer_list {
 //   4. A full border node below a parent with room is split in the same way.
 // What does not fit (roots and parents to be split, entries that become new
 // layers, nodes that stay locked) goes to the defer list.
-// A pair of 1M mixed batches on 16M keys: 2.72 ms, from 4.94 ms with one
-// kernel per class and 32 lanes per write (1,505 warp instructions and two
-// fences per insert; now about 500, and the fences serve 32 requests); insert +
-// update + find + erase of 300K keys each on 4M keys 1.58 -> 0.65 ms.
-// 1M finds (half of them misses) on 1M keys of 1-8 slices: 235 us, from
-// 357 us with eight lanes per request (55 warp instructions per find instead
-// of 587).  What bounds it now: a lane's 32-byte loads touch 32 lines per
-// instruction, so the load path moves one sector per cycle (62% busy); the
-// occupancy (4, 6 or 8 blocks per SM) changes nothing.
+// Measured against tiles of 8 lanes per find and 32 per write: a pair of 1M
+// mixed batches on 16M keys 1.18 ms (4.94), insert + update + find + erase of
+// 300K keys each on 4M keys 0.45 ms (1.57), 1M finds (half of them misses) on 1M
+// keys of 1-8 slices 120 us (357; 70 warp instructions per find instead of 587).
+// Finds are bound by the load path (64% busy: every node goes through shared
+// memory as one line) and by issue (51%); mixed batches by the latency of up to
+// 17 dependent node visits and two fences per round, with about 4 warps per
+// scheduler: at 3, 4, 5 and 6 blocks per SM they differ by less than 4%.
 template <int OP, bool CONC, class Src>
 MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl) {
   constexpr uint32_t kAll = 0xFFFFFFFFu;

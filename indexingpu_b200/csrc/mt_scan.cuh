@@ -5,7 +5,11 @@
 // (mt_node.cuh), so the results of a border node are written side by side: each
 // lane reads its own entry's chain line and writes its own output row.  (With
 // one entry after the other, as coop_scan does, a query waits for 13 chain
-// lines per node in turn.)
+// lines per node in turn.)  400K queries of 100 results on 32M keys: 2.01 ms,
+// from 5.25 ms with one entry after the other on 4 lanes (2.30 before the bulk
+// build laid neighbours' chains side by side); bound by random 128-byte lines,
+// of which a result uses a few words.  At 8 blocks per SM; 6 take 2.54 and 10
+// take 2.77 ms, and asking L2 for the next node's chains changes nothing.
 #pragma once
 #include "mt_internal.cuh"
 
