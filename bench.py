@@ -383,8 +383,8 @@ def run_ours(args, rank, world, dist):
                        "preload_keys": args.preload, "batch_requests": args.batch, "max_key_length": MAXK,
                        "max_value_length": MAXV, "tile_size": args.tile, "write_tile_size": args.write_tile,
                        "upderase_tile_size": args.upderase_tile or args.write_tile,
-                       "form": "plain per-call mixed_batch (reclaim, three-way partition, find / insert / "
-                               "update+erase class kernels on forked streams, updates of one key combined)",
+                       "form": "plain per-call mixed_batch (reclaim, update combining, one request per lane, tile kernel "
+                               "for the rest, results of combined updates)",
                        "l2": "no flush: the index (>2 GB of slabs) and each batch's inputs exceed the 126 MB L2",
                        "parallelism": f"replicas x{world}"},
             "batch_latency_ms": {"p50": round(sorted_steps[len(sorted_steps) // 2], 4),
@@ -399,7 +399,7 @@ def run_ours(args, rank, world, dist):
                          "frac": round(achieved / peak, 4), "peak_source": peak_kind,
                          "traffic": None if tr is None else int(tr * args.batch),
                          "algorithmic_bytes_per_step": abytes // args.steps,
-                         "kernel": "mixed_batch call: reclaim + partition + three class kernels"},
+                         "kernel": "mixed_batch call: reclaim + combining + lane kernel + rest"},
             "cpu_baseline": cpu,
             "clocks": clk,
             # reclaim, partition, find class, insert class, update combining,
