@@ -125,3 +125,39 @@ def test_writes_that_meet_in_one_node(upsert):
         _same_contents(g, o, 3 * n, 1, 1)
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("n", [2, 255, 256, 257, 1025, 303104, 303105, 310000])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_updates_of_one_key_in_one_call(n, mixed):
+    # Chunks of 256 and of 1,024 requests per block, whole and ragged; a call
+    # after smaller and larger ones (the table keeps the entries of earlier
+    # calls).  Updates of one key have no order: the result is every request's,
+    # the value one of theirs.
+    g = GpuIndex(pool_bytes=64 << 20)
+    rng = np.random.default_rng(n)
+    held = 5000
+    try:
+        keys = np.stack([np.arange(held), np.arange(held) % 7], 1).astype(np.uint32)
+        two, one = np.full(held, 2, np.uint32), np.ones(held, np.uint32)
+        assert g.insert(keys, two, np.zeros((held, 1), np.uint32), one).all()
+        for size in (n, 3, n):
+            ids = rng.integers(0, held + 50, size)
+            k = np.stack([ids, ids % 7], 1).astype(np.uint32)
+            v = (np.arange(size, dtype=np.uint32) + 1)[:, None]
+            l2, l1 = np.full(size, 2, np.uint32), np.ones(size, np.uint32)
+            if mixed:
+                types = np.where(np.arange(size) % 3 == 0, 2, 3).astype(np.uint8)
+                res = np.array(g.mixed(types, k, l2, v, l1)[2])
+                upd = types == 3
+            else:
+                res, upd = np.array(g.update(k, l2, v, l1)), np.ones(size, bool)
+            np.testing.assert_array_equal(res[upd] != 0, ids[upd] < held)
+            got, gl = g.find(keys, two, 1)
+            assert (gl == 1).all()
+            touched = np.unique(ids[upd & (ids < held)])
+            written = got[touched, 0].astype(np.int64) - 1
+            assert (ids[written] == touched).all() and upd[written].all()
+            g.update(keys, two, np.zeros((held, 1), np.uint32), one)
+    finally:
+        g.close()
