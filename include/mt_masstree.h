@@ -105,8 +105,8 @@ typedef struct mt_stats_t {
 
 /* Construction.  Replaces gpu_masstree(allocator(pool_ratio), reclaimer())
  * (reference gpu_masstree.hpp:67-72, simple_slab_alloc.hpp:56-69): the slab
- * pool takes pool_ratio of the currently free device memory (a little is
- * allocated beside it: counters and a list of at most 1/256 of the pool).
+ * pool takes pool_ratio of the currently free device memory (a few KB of
+ * counters are allocated beside it).
  * tile_size: see mt_set_tile_size. */
 int mt_create(mt_masstree** out, float pool_ratio, uint32_t tile_size);
 /* Same, with the pool size given in bytes. */
@@ -116,8 +116,7 @@ int mt_destroy(mt_masstree* tree);
 
 /* Launch shape: lanes per request (4/8/16/32) of the kernels that serve a
  * request with a tile of lanes (serving loop, MT_FLAG_PERSISTENT,
- * MT_FLAG_SINGLE_PASS, mt_mixed_batch_noalloc's writes, and the requests that
- * the one-request-per-lane kernels of the batch calls hand on), and resident
+ * MT_FLAG_SINGLE_PASS and mt_mixed_batch_noalloc's writes), and resident
  * blocks per SM (0 = as many as fit).  The batch calls themselves serve one
  * request per lane, scans 16 lanes per query, whatever the width.  New in this
  * library. */
@@ -224,9 +223,8 @@ int mt_batches_reserve(mt_masstree* tree, uint32_t max_subbatches, uint64_t max_
 
 /* Serve num_subbatches mixed batches in order, with the results of one
  * mt_mixed_batch call per sub-batch: sub-batch k+1 sees every effect of
- * sub-batch k.  By default each sub-batch is one kernel, one request per lane,
- * and a second one for the few requests that the first hands on; with
- * MT_FLAG_PERSISTENT a partition pass files every request of every sub-batch
+ * sub-batch k.  By default each sub-batch is one kernel, one request per lane;
+ * with MT_FLAG_PERSISTENT a partition pass files every request of every sub-batch
  * under its class and one cooperative persistent launch serves all
  * sub-batches with a grid barrier between them.  `subbatches` is a DEVICE
  * array of descriptors; nothing is read back to the host and the number of

@@ -1,9 +1,8 @@
 """Autotuner for the batched form (mt_mixed_batches).
 
 Searches the form and launch shape of the call over
-  form ("forked": a lane kernel per sub-batch and a tile kernel for what it
-  hands on; one persistent launch for all sub-batches; or all sub-batches at
-  once grouped by key) x
+  form ("forked": a lane kernel per sub-batch; one persistent launch for all
+  sub-batches; or all sub-batches at once grouped by key) x
   find tile (lanes per find: 4, 8, 16, 32) x write tile (lanes per insert,
   update and erase: 16, 32) x key-length bucketing (off, on; the grouped
   form has no buckets and runs once per tile pair),

@@ -12,8 +12,7 @@
 //   3. (MT_FLAG_PERSISTENT) batches_persistent_kernel: a cooperative grid walks
 //      the sub-batches in order with one grid barrier between sub-batches;
 //   or, by default, instead of 2 and 3: for every sub-batch one kernel that
-//      serves its requests one per lane (mt_lane.cuh), and a tile kernel for
-//      the few it hands on.
+//      serves its requests one per lane (mt_lane.cuh).
 // Sub-batch k+1 observes every effect of sub-batch k, as with one host call per
 // sub-batch; inside a sub-batch the classes have no order among each other
 // (as inside one mixed batch).  Nothing in the call allocates once
@@ -146,9 +145,7 @@ __global__ void __launch_bounds__(kBlock, MT_MIN_BLOCKS_PER_SM) batches_persiste
   wcache.release(tw, tv.pool);
 }
 
-// Default form: the requests of one sub-batch, one per lane, and then those
-// that the lanes handed on (their list is the sub-batch's part of lists, its
-// count the first of the sub-batch's counters).
+// Default form: the requests of one sub-batch, one per lane.
 MT_DEV batch_args subbatch_args(const batches_view& b, uint32_t sb) {
   batch_args a = class_args(b, sb, 0u);
   a.index = nullptr;
@@ -159,25 +156,8 @@ MT_DEV batch_args subbatch_args(const batches_view& b, uint32_t sb) {
 __global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) batches_lane_kernel(tree_view tv, batches_view b,
                                                                                     uint32_t sb) {
   if (b.status[0]) return;
-  const defer_list dl{b.lists + b.offsets[sb], b.counts + sb * kCountStride};
-  lane_serve<OP_MIXED, true>(tv, batch_source{subbatch_args(b, sb)}, dl);
+  lane_serve<OP_MIXED, true>(tv, batch_source{subbatch_args(b, sb)});
 }
-template <int T>
-__global__ void __launch_bounds__(kBlock, MT_MIN_BLOCKS_PER_SM) batches_rest_kernel(tree_view tv, batches_view b,
-                                                                                    uint32_t sb) {
-  if (b.status[0]) return;
-  tile<T> t;
-  const uint32_t tile_id = (blockIdx.x * blockDim.x + threadIdx.x) / T;
-  const uint32_t num_tiles = (gridDim.x * blockDim.x) / T;
-  slab_cache<T> cache;
-  cache.init(tv.pool, tile_id);
-  batch_args a = subbatch_args(b, sb);
-  a.index = b.lists + b.offsets[sb];
-  a.n_dev = b.counts + sb * kCountStride;
-  serve_requests<T, OP_MIXED, true>(t, tv, cache, a, tile_id, num_tiles);
-  cache.release(t, tv.pool);
-}
-
 }  // namespace mtb
 
 using namespace mtb;
@@ -186,21 +166,12 @@ namespace {
 
 int launch_status() { return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA; }
 
-template <int T>
-int launch_rest(mt_masstree* t, const batches_view& b, uint32_t sb, cudaStream_t s) {
-  int bps = host_max_blocks_per_sm((const void*)batches_rest_kernel<T>, kBlock, 0);
-  if (t->blocks_per_sm > 0) bps = std::min<int>(bps, (int)t->blocks_per_sm);
-  batches_rest_kernel<T><<<std::max(bps, 1) * t->sms, kBlock, 0, s>>>(t->tv, b, sb);
-  return launch_status();
-}
-
 // The sub-batches' sizes are on the device only: the grids fill the GPU.
 int launch_each(mt_masstree* t, const batches_view& b, cudaStream_t s) {
   const int grid = host_lane_grid(t, (const void*)batches_lane_kernel, b.max_total);
   for (uint32_t sb = 0; sb < b.nsub; ++sb) {
     batches_lane_kernel<<<grid, kBlock, 0, s>>>(t->tv, b, sb);
-    int rc = launch_status();
-    if (!rc) rc = t->write_tile_size <= 16 ? launch_rest<16>(t, b, sb, s) : launch_rest<32>(t, b, sb, s);
+    const int rc = launch_status();
     if (rc) return rc;
   }
   return MT_OK;

@@ -1,10 +1,10 @@
 // Batch kernels and the C ABI of libmt_b200.so.
 //
 // A host call is a short, fixed sequence of stream-ordered launches: the reclaim
-// pass that returns slabs retired by earlier calls (not for finds), a
-// grid-stride kernel that serves one request per lane (mt_lane.cuh), and a tile
-// kernel for the requests that it hands on (the reference launches one tile
-// kernel, include/kernels.hpp:31-103).  Differences:
+// pass that returns slabs retired by earlier calls (not for finds) and a
+// grid-stride kernel that serves one request per lane (mt_lane.cuh; the
+// reference's kernel serves one per tile, include/kernels.hpp:31-103).
+// Differences:
 //   * the launch shape (blocks per SM from the occupancy API, SM count) is
 //     computed once per kernel and cached, not on every call (the reference
 //     queries it per call, kernels.hpp:91-99);
@@ -160,14 +160,14 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for<OP>) batch_kernel(tree_
 
 template <bool CONC>
 __global__ void __launch_bounds__(kBlock, MT_LANE_FIND_BLOCKS) find_kernel(tree_view tv, batch_args a) {
-  lane_serve<OP_FIND, CONC>(tv, batch_source{a}, defer_list{nullptr, nullptr});
+  lane_serve<OP_FIND, CONC>(tv, batch_source{a});
 }
 
 // Inserts, updates, erases and mixed batches, one request per lane (what bounds
 // them and what they measured: lane_serve).
 template <int OP>
-__global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) lane_kernel(tree_view tv, batch_args a, defer_list dl) {
-  lane_serve<OP, true>(tv, batch_source{a}, dl);
+__global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) lane_kernel(tree_view tv, batch_args a) {
+  lane_serve<OP, true>(tv, batch_source{a});
 }
 
 template <bool CONC>
@@ -263,12 +263,9 @@ __global__ void line_atomicity_kernel(uint32_t* lines, uint32_t nlines, uint32_t
 }
 
 // Return slabs retired by earlier launches to their shard's free stack; start
-// the call's defer list empty (call[0]) and its epoch (call[1]).
-__global__ void reclaim_kernel(pool_view p, uint32_t* call) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    call[0] = 0u;
-    call[1] += 1u;
-  }
+// the call's epoch.
+__global__ void reclaim_kernel(pool_view p, uint32_t* epoch) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *epoch += 1u;
   for (uint32_t s = blockIdx.x; s < p.num_shards; s += gridDim.x) {
     __shared__ int top, n;
     if (threadIdx.x == 0) {
@@ -302,7 +299,7 @@ int host_max_blocks_per_sm(const void* fn, int block, size_t smem) {
   return b;
 }
 int host_launch_reclaim(mt_masstree* t, cudaStream_t s) {
-  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->defer_mem);
+  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->epoch);
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
 }
 }  // namespace mtb
@@ -356,7 +353,7 @@ namespace {
 int cuda_status(cudaError_t e) { return e == cudaSuccess ? MT_OK : MT_ERR_CUDA; }
 
 int launch_reclaim(mt_masstree* t, cudaStream_t s) {
-  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->defer_mem);
+  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->epoch);
   return cuda_status(cudaGetLastError());
 }
 
@@ -378,33 +375,18 @@ int launch_batch_tile(mt_masstree* t, uint32_t tile, const batch_args& a, cudaSt
   }
 }
 
-// Writes and mixed batches: the lane kernel, then a tile kernel for the
-// requests it hands on (few: splits of roots and full parents, new layers,
-// nodes under contention), in pieces that fit the defer list.
-// The reclaim pass is the caller's.
+// Writes and mixed batches, one request per lane.  The reclaim pass is the
+// caller's.
 template <int OP>
-int launch_lane(mt_masstree* t, batch_args a, uint32_t tile, cudaStream_t s) {
-  int rc = MT_OK;
-  const defer_list dl{t->defer_mem + 32, t->defer_mem};
-  const uint32_t n = a.n;
-  for (uint32_t first = 0; !rc && first < n; first += a.n) {
-    a.first = first;
-    a.n = std::min(n - first, t->defer_cap);
-    if (first && cudaMemsetAsync(dl.count, 0, sizeof(uint32_t), s) != cudaSuccess) return MT_ERR_CUDA;
-    lane_kernel<OP><<<host_lane_grid(t, (const void*)lane_kernel<OP>, a.n), kBlock, 0, s>>>(t->tv, a, dl);
-    if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
-    batch_args d = a;
-    d.index = dl.list;
-    d.n_dev = dl.count;
-    rc = launch_batch_tile<OP, true>(t, tile, d, s);
-  }
-  return rc;
+int launch_lane(mt_masstree* t, const batch_args& a, cudaStream_t s) {
+  lane_kernel<OP><<<host_lane_grid(t, (const void*)lane_kernel<OP>, a.n), kBlock, 0, s>>>(t->tv, a);
+  return cuda_status(cudaGetLastError());
 }
 template <int OP>
 int launch_writes(mt_masstree* t, const batch_args& a, cudaStream_t s) {
   if (a.n == 0) return MT_OK;
   const int rc = launch_reclaim(t, s);
-  return rc ? rc : launch_lane<OP>(t, a, t->write_tile_size, s);
+  return rc ? rc : launch_lane<OP>(t, a, s);
 }
 
 // Finds take no slabs, so no reclaim pass precedes them.  a.n: the number of
@@ -455,7 +437,7 @@ int launch_combine(mt_masstree* t, batch_args& a, cudaStream_t s) {
   const uint32_t mask = combine_slots(a.n) - 1u;  // a small call stays within a small part of the table
   const uint32_t chunk = a.n <= (uint32_t)t->sms * 8u * kCombineThreads ? kCombineThreads : kCombineChunk;
   const int grid = std::max(1, std::min<int>(t->sms * 8, (int)(a.n / chunk + (a.n % chunk != 0u))));
-  combine_kernel<<<grid, kCombineThreads, 0, s>>>(a, table, mask, leader_of, t->defer_mem + 1, chunk);
+  combine_kernel<<<grid, kCombineThreads, 0, s>>>(a, table, mask, leader_of, t->epoch, chunk);
   if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
   a.leader_of = leader_of;
   return MT_OK;
@@ -474,7 +456,7 @@ int launch_mixed(mt_masstree* t, batch_args a, cudaStream_t s) {
   int rc = ensure_combine_scratch(t, a.n, s);
   if (!rc) rc = launch_reclaim(t, s);
   if (!rc) rc = launch_combine(t, a, s);
-  if (!rc) rc = launch_lane<OP_MIXED>(t, a, t->write_tile_size <= 16 ? 16u : 32u, s);
+  if (!rc) rc = launch_lane<OP_MIXED>(t, a, s);
   if (!rc) rc = launch_combine_results(t, a, a.n, s);
   return rc;
 }
@@ -521,10 +503,8 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
   const size_t stack_bytes = nslabs * 4u;
   const size_t ctr_bytes = (size_t)kShards * 3u * kCtrStride * sizeof(int);
   const size_t err_bytes = 128;
-  // The defer list of the lane kernels: 1/256 of the pool, at most 16M entries
-  // (a call of more requests is served in pieces, each with its own tail).
-  const uint64_t defer_cap = std::min<uint64_t>(1u << 24, std::max<uint64_t>(4096u, pool_bytes / 1024u));
-  const size_t total = slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes + 128 + defer_cap * 4u;
+  const size_t epoch_bytes = 128;
+  const size_t total = slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes + epoch_bytes;
   if (cudaMalloc(&t->mem, total) != cudaSuccess) { delete t; return MT_ERR_OOM; }
   char* base = (char*)t->mem;
   pool_view& p = t->tv.pool;
@@ -533,13 +513,12 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
   p.limbo = (uint32_t*)(base + slab_bytes + stack_bytes);
   p.ctr = (int*)(base + slab_bytes + 2 * stack_bytes);
   p.err = (uint32_t*)(base + slab_bytes + 2 * stack_bytes + ctr_bytes);
-  t->defer_mem = (uint32_t*)(base + slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes);
-  t->defer_cap = (uint32_t)defer_cap;
+  t->epoch = (uint32_t*)(base + slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes);
   p.num_slabs = (uint32_t)nslabs;
   p.num_shards = kShards;
   p.shard_slabs = shard_slabs;
   p.lock_spins = kLockSpins;
-  cudaError_t e = cudaMemset(p.ctr, 0, ctr_bytes + err_bytes + 128);  // and the call words in front of the defer list
+  cudaError_t e = cudaMemset(p.ctr, 0, ctr_bytes + err_bytes + epoch_bytes);
   // Root of trie layer 0 = slab 0 (shard 0's bump pointer starts past it).
   uint32_t root_img[32] = {0};
   root_img[WORD_HIGH] = 0xFFFFFFFFu;
@@ -707,7 +686,7 @@ int mt_update(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_
   int rc = ensure_combine_scratch(t, n, s);
   if (!rc) rc = launch_reclaim(t, s);
   if (!rc) rc = launch_combine(t, a, s);
-  if (!rc) rc = launch_lane<OP_UPDATE>(t, a, t->write_tile_size, s);
+  if (!rc) rc = launch_lane<OP_UPDATE>(t, a, s);
   if (!rc) rc = launch_combine_results(t, a, n, s);
   return rc;
 }

@@ -81,9 +81,7 @@ struct grouped_view {
   uint32_t* heads;           // run heads of keys touched more than once (count: counts[0])
   uint32_t* singles;         // requests on keys touched once (count: counts[1])
   uint32_t* serial;          // heads of runs served one by one (count: counts[2])
-  uint32_t* rest;            // singles left to the tile kernel (count: counts[3])
-  uint32_t* rest_heads;      // final writes left to the tile kernel (count: counts[4])
-  uint32_t* counts;          // [5], zeroed at the start of the call
+  uint32_t* counts;          // [3], zeroed at the start of the call
   unsigned long long hash_mask;  // bits of the key hash used (mt_set_group_hash_bits)
 };
 
@@ -262,7 +260,7 @@ struct group_first_source {
   }
 };
 __global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) group_first_kernel(tree_view tv, grouped_view g) {
-  lane_serve<OP_MIXED, true>(tv, group_first_source{g}, defer_list{g.rest, &g.counts[3]});
+  lane_serve<OP_MIXED, true>(tv, group_first_source{g});
 }
 
 // 6. Results of the requests on keys touched more than once, from the scanned
@@ -332,41 +330,7 @@ struct group_final_source {
   MT_DEV void result(uint32_t, const lane_request&, bool) const {}
 };
 __global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) group_final_kernel(tree_view tv, grouped_view g) {
-  lane_serve<OP_MIXED, true>(tv, group_final_source{g}, defer_list{g.rest_heads, &g.counts[4]});
-}
-
-// What the lanes handed on: HEADS, final writes, else requests on keys touched
-// once (never finds).
-template <int T, bool HEADS>
-__global__ void __launch_bounds__(kBlock, MT_WRITE_MIN_BLOCKS_PER_SM) group_rest_kernel(tree_view tv, grouped_view g) {
-  tile<T> t;
-  const uint32_t tile_id = (blockIdx.x * blockDim.x + threadIdx.x) / T;
-  const uint32_t num_tiles = (gridDim.x * blockDim.x) / T;
-  slab_cache<T> cache;
-  cache.init(tv.pool, tile_id);
-  const uint32_t n = g.counts[HEADS ? 4 : 3];
-  for (uint32_t k = tile_id; k < n; k += num_tiles) {
-    if (t.shfl((uint32_t)(t.leader() && fatal_error(tv.pool)), 0)) break;
-    const uint32_t j = HEADS ? g.rest_heads[k] : g.rest[k];
-    const greq r = group_req(g, g.gid[j]);
-    const uint32_t* key = greq_key(g, r);
-    greq w = r;
-    uint32_t kind = r.kind;
-    if (HEADS) {
-      const uint32_t act = g.act[j];
-      kind = MT_REQ_ERASE;
-      if (act != kGAbsent) {
-        w = group_req(g, act);
-        kind = g.init[j] == kGAbsent ? MT_REQ_INSERT : MT_REQ_UPDATE;
-      }
-    }
-    int res;
-    if (kind == MT_REQ_INSERT) res = coop_insert<T, false>(t, tv, cache, key, r.klen, greq_val(g, w), w.vlen);
-    else if (kind == MT_REQ_UPDATE) res = coop_update<T>(t, tv, cache, key, r.klen, greq_val(g, w), w.vlen);
-    else res = coop_erase<T>(t, tv, key, r.klen);
-    if (!HEADS && t.leader() && r.d->results) r.d->results[r.i] = res == RES_OK;
-  }
-  cache.release(t, tv.pool);
+  lane_serve<OP_MIXED, true>(tv, group_final_source{g});
 }
 
 // 8. Runs holding two keys under one hash: every request in order.
@@ -426,7 +390,7 @@ int ensure_grouped(mt_masstree* t, uint32_t m, uint32_t max_v, cudaStream_t s) {
                                           hash_equal(), s) != cudaSuccess)
     return MT_ERR_CUDA;
   const size_t temp = std::max(sort_bytes, scan_bytes);
-  const size_t bytes = 4 * up256((size_t)m * 8u) + 2 * up256((size_t)m * sizeof(gfn)) + 8 * up256((size_t)m * 4u) +
+  const size_t bytes = 4 * up256((size_t)m * 8u) + 2 * up256((size_t)m * sizeof(gfn)) + 6 * up256((size_t)m * 4u) +
                        up256((size_t)m * max_v * 4u) + up256(temp);
   if (cudaDeviceSynchronize() != cudaSuccess) return MT_ERR_CUDA;
   if (t->grouped_mem) cudaFree(t->grouped_mem);
@@ -459,14 +423,12 @@ int launch_lanes(mt_masstree* t, void (*fn)(tree_view, grouped_view), const grou
 template <int TW>
 int launch_served(mt_masstree* t, const grouped_view& g, cudaStream_t s) {
   int rc = launch_lanes(t, group_first_kernel, g, s);
-  if (!rc) rc = launch_tile_kernel<TW>(t, group_rest_kernel<TW, false>, g, s);
   if (!rc) rc = launch_tile_kernel<TW>(t, group_serial_kernel<TW>, g, s);
   if (rc) return rc;
   const int grid = std::max(1, std::min<int>(t->sms * 8, (int)((g.m + 255u) / 256u)));
   group_result_kernel<<<grid, 256, 0, s>>>(g);
   if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
   rc = launch_lanes(t, group_final_kernel, g, s);
-  if (!rc) rc = launch_tile_kernel<TW>(t, group_rest_kernel<TW, true>, g, s);
   return rc;
 }
 
@@ -506,11 +468,9 @@ int launch_grouped(mt_masstree* t, const batches_view& b, cudaStream_t s) {
   g.heads = reinterpret_cast<uint32_t*>(carve(M * 4u));
   g.singles = reinterpret_cast<uint32_t*>(carve(M * 4u));
   g.serial = reinterpret_cast<uint32_t*>(carve(M * 4u));
-  g.rest = reinterpret_cast<uint32_t*>(carve(M * 4u));
-  g.rest_heads = reinterpret_cast<uint32_t*>(carve(M * 4u));
   void* temp = carve(t->grouped_temp);
   g.counts = b.status + 2;
-  if (cudaMemsetAsync(g.counts, 0, 5 * sizeof(uint32_t), s) != cudaSuccess) return MT_ERR_CUDA;
+  if (cudaMemsetAsync(g.counts, 0, 3 * sizeof(uint32_t), s) != cudaSuccess) return MT_ERR_CUDA;
   const int grid = std::max(1, std::min<int>(t->sms * 8, (int)((m + 255u) / 256u)));
   group_hash_kernel<<<grid, 256, 0, s>>>(t->tv, g, hash_in, gid_in);
   if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;

@@ -68,7 +68,6 @@ struct batch_args {
   uint32_t max_key_length;
   uint32_t max_value_length;
   uint32_t n;
-  uint32_t first;              // lane kernels: serve requests (or index entries) first .. first + n
 };
 
 struct scan_args {
@@ -229,8 +228,7 @@ struct mt_masstree {
   uint32_t blocks_per_sm = 0;    // 0 = occupancy limit
   uint32_t* combine_mem = nullptr;  // update-combining scratch (grown on demand)
   uint32_t combine_cap = 0;
-  uint32_t* defer_mem = nullptr;    // requests the lane kernels hand on: count (one line), then defer_cap entries
-  uint32_t defer_cap = 0;
+  uint32_t* epoch = nullptr;        // number of the call in the combining table (device)
   mt_host_pipe* host_pipe = nullptr;
   void* mem = nullptr;
   mtb::tree_view tv{};

@@ -1,11 +1,13 @@
 // One request per thread: the batch kernels' way through the tree.
 //
-// A lane walks its request's path alone, with the whole 128-byte node in its
-// registers (four 32-byte loads), so a warp has 32 independent walks in flight
-// where the tile code (mt_tree.cuh) has 32 / T, and a node visit costs no
-// shuffle, vote or reduction.  What benefits from neighbouring lanes reading
-// neighbouring words (suffix chains, key rests, values) is done by eight lanes
-// per request, four requests at a time (warp_chains).
+// A lane walks its request's path alone: eight lanes bring the node to the
+// lane's line of shared memory, the lane searches it in its registers.  So a
+// warp has 32 independent walks in flight where the tile code (mt_tree.cuh) has
+// 32 / T, and a node visit costs no vote or reduction.  What benefits from
+// neighbouring lanes reading neighbouring words (suffix chains, key rests,
+// values) is done by eight lanes per request, four requests at a time
+// (warp_chains).  The few requests that need more than one node and its parent
+// are served by the whole warp as one tile.
 #pragma once
 #include "mt_internal.cuh"
 
@@ -16,7 +18,9 @@ namespace mtb {
 // as any (B-link nodes are never unlinked while a launch runs, so a stale
 // interior node still leads to its key through sibling links, and requests of
 // one batch have no order), and the checksum rejects a torn one, which is then
-// read again from L2.  The upper levels of the tree, which every request
+// read again from L2.  A node that was split again and again since its parent
+// came to L1 would be a long way from its last half: after kMaxSideways moves
+// the walk starts its layer again, from L2.  The upper levels of the tree, which every request
 // passes, thus come from L1 (reading them all from L2 costs a pair of 1M mixed
 // batches 3.39 instead of 2.79 ms).
 MT_DEV void lane_load_relaxed(const uint32_t* a, uint32_t (&w)[32]) {
@@ -137,8 +141,11 @@ struct lane_place {
   uint32_t state;   // the entry's key state
   uint32_t val;     // the entry's value word
   bool found;
-  bool full;        // the border node has no room (and is not a layer root)
+  bool full;        // the border node has no room
+  bool stuck;       // and is a root, or its parent has no room either: only a tile can split it
 };
+
+constexpr uint32_t kMaxSideways = 8;
 
 // Walk from the root of layer 0 to the key's place, for the lanes with `go`
 // (klen > 0); called by the whole warp.  The warp goes round the loop together,
@@ -148,7 +155,9 @@ struct lane_place {
 template <bool CONC>
 MT_DEV void lane_locate(const tree_view& tv, bool& go, const uint32_t* key, uint32_t klen, lane_place& at) {
   const pool_view& p = tv.pool;
-  uint32_t idx = tv.root, hops = 0, torn = 0;
+  uint32_t idx = tv.root, hops = 0, torn = 0, sideways = 0;
+  bool parent_full = true;  // (or there is none)
+  bool from_l2 = false;
   uint32_t slice = go ? key[0] : 0u;
   bool more = klen > 1u;
   bool walk = go;
@@ -160,14 +169,14 @@ MT_DEV void lane_locate(const tree_view& tv, bool& go, const uint32_t* key, uint
 #pragma unroll 1
   while (__any_sync(0xFFFFFFFFu, walk)) {
     const bool ok = p.valid(idx);
-    warp_load_nodes(p, lines, walk && ok && torn == 0u, idx);
+    warp_load_nodes(p, lines, walk && ok && torn == 0u && !from_l2, idx);
     if (walk) {
       uint32_t err = ERR_NONE;
       if (!ok || ++hops > kMaxHops) {
         err = ERR_CORRUPT;
       } else {
         uint32_t w[32];
-        if (CONC && torn != 0u) lane_load_relaxed(p.addr(idx), w);
+        if (CONC && (torn != 0u || from_l2)) lane_load_relaxed(p.addr(idx), w);
         else lane_take_line(lines, w);
         if (CONC && !lane_verify(w)) {  // read again, from L2 (bounded, as node::load_verified)
           --hops;
@@ -180,8 +189,15 @@ MT_DEV void lane_locate(const tree_view& tv, bool& go, const uint32_t* key, uint
           const uint32_t pos = lane_search(w, slice, more, k, v);
           if ((meta & META_SIB) && slice > w[WORD_HIGH]) {
             idx = w[WORD_SIB];
+            if (CONC && ++sideways > kMaxSideways && !from_l2) {
+              from_l2 = true;
+              idx = at.root;
+              at.parent = kInvalid;
+              parent_full = true;
+            }
           } else if (!border) {
             at.parent = idx;
+            parent_full = (meta & META_COUNT) >= (uint32_t)kMaxEntries;
             idx = pos < (meta & META_COUNT) ? v : kInvalid;  // none: caught as an invalid slab above
           } else {
             const uint32_t state = ks_get(w[WORD_KS], pos);
@@ -190,12 +206,14 @@ MT_DEV void lane_locate(const tree_view& tv, bool& go, const uint32_t* key, uint
               idx = v;
               at.root = v;
               at.parent = kInvalid;
+              parent_full = true;
               ++at.layer;
               slice = key[at.layer];
               more = at.layer + 1u < klen;
             } else {
               at.idx = idx;
-              at.full = (meta & (META_COUNT | META_ROOT)) == (uint32_t)kMaxEntries;
+              at.full = (meta & META_COUNT) >= (uint32_t)kMaxEntries;
+              at.stuck = at.full && ((meta & META_ROOT) || parent_full);
               at.found = hit;
               at.state = state;
               at.val = v;
@@ -335,7 +353,7 @@ MT_DEV uint32_t lane_slot(uint32_t lane) { return (lane & 7u) * 4u + (lane >> 3)
 // One request as a lane serves it.  `val`: the value rows of inserts and
 // updates (input) and finds (output; may be null).
 struct lane_request {
-  uint32_t id;  // what the defer list gets
+  uint32_t id;
   uint32_t kind, klen, vlen;
   const uint32_t* key;
   uint32_t* val;
@@ -352,7 +370,7 @@ struct batch_source {
   MT_DEV uint32_t max_value_length() const { return a.max_value_length; }
   template <int OP>
   MT_DEV uint32_t fetch(const pool_view& p, uint32_t pos, lane_request& r) const {
-    const uint32_t i = a.index ? a.index[a.first + pos] : a.first + pos;
+    const uint32_t i = a.index ? a.index[pos] : pos;
     r.id = i;
     r.kind = MT_REQ_FIND;
     if (OP == OP_MIXED) r.kind = a.types[i];
@@ -403,8 +421,8 @@ MT_DEV void lane_store_weak(uint32_t* a, const uint32_t (&w)[32]) {
 }
 
 // Attempts of a lane on its border node (each one a read and perhaps an
-// atomic) before the request goes to the tile kernel that follows, which
-// waits for locks, splits roots and full parents, and makes new layers.
+// atomic) before the whole warp serves the request as a tile, which waits for
+// locks, splits roots and full parents, and makes new layers.
 constexpr uint32_t kLaneTries = 24;
 
 // Slabs that a warp took together; one lane's are the positions
@@ -422,13 +440,24 @@ MT_DEV uint32_t lane_slab(const pool_view& p, const lane_slabs& s, uint32_t q) {
   return s.shard * p.shard_slabs + s.bump + (k - s.n_stack);
 }
 
+// Keep a chain of n slabs that nothing leads to in the warp's slab cache (one lane).
+MT_DEV void lane_keep_slabs(const pool_view& p, uint32_t head, uint32_t n, slab_cache<32>& cache) {
+  uint32_t tail = head;
+#pragma unroll 1
+  for (uint32_t q = 1; q < n; ++q) tail = ld_relaxed_u32(p.addr(tail) + kNextWord);
+  st_relaxed_u32(p.addr(tail) + kNextWord, cache.vain);
+  cache.vain = head;
+  cache.vain_n += n;
+}
+
 // Take `need` slabs for every lane of the warp (0: none): one atomic or two
 // for the whole warp per shard asked.  A shard that cannot serve everyone
 // serves the first lanes; the next shards serve the others.  Returns whether
-// the lane got its slabs (no error is recorded: the caller hands the request
-// on).
-MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, uint32_t& shard, lane_slabs& s) {
+// the lane got its slabs (no error is recorded: a tile, which takes one slab
+// after the other from any shard, serves the request then).
+MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, slab_cache<32>& cache, lane_slabs& s) {
   const uint32_t lane = lane_id();
+  uint32_t& shard = cache.shard;
   bool got = need == 0u;
 #pragma unroll 1
   for (uint32_t k = 0; k < p.num_shards; ++k) {
@@ -441,11 +470,16 @@ MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, uint32_t& shard, 
     }
     const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
     if (total == 0u) break;
+    // A shard that cannot cover the first lane's need is left as it is.
+    const uint32_t least = __shfl_sync(0xFFFFFFFFu, want, __ffs(__ballot_sync(0xFFFFFFFFu, want != 0u)) - 1);
     int lo = 0, n_stack = 0, bump = 0, n_bump = 0;
     if (lane == 0u) {
-      int left = (int)total;
       int* topp = p.top(shard);
-      if ((int)ld_relaxed_u32((const uint32_t*)topp) > 0) {
+      int* bp = p.bump(shard);
+      const int on_stack = max((int)ld_relaxed_u32((const uint32_t*)topp), 0);
+      const int above = max((int)p.shard_slabs - (int)ld_relaxed_u32((const uint32_t*)bp), 0);
+      int left = (uint32_t)(on_stack + above) >= least ? (int)total : 0;
+      if (left > 0 && on_stack > 0) {
         const int old = atomicSub(topp, left);
         if (old > 0) {
           lo = max(old - left, 0);
@@ -453,8 +487,7 @@ MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, uint32_t& shard, 
           left -= n_stack;
         }
       }
-      int* bp = p.bump(shard);
-      if (left > 0 && (int)ld_relaxed_u32((const uint32_t*)bp) < (int)p.shard_slabs) {
+      if (left > 0 && above > 0) {
         const int b = atomicAdd(bp, left);
         if (b < (int)p.shard_slabs) {
           bump = b;
@@ -478,9 +511,12 @@ MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, uint32_t& shard, 
         s = g;
         got = true;
       } else {
-        // The part of a lane's need that this shard covered goes back.
+        // The part of a lane's need that this shard covered stays with the warp.
 #pragma unroll 1
-        for (uint32_t q = g.first; q < have; ++q) retire_slab(p, lane_slab(p, g, q - g.first));
+        for (uint32_t q = g.first; q < have; ++q) {
+          const uint32_t x = lane_slab(p, g, q - g.first);
+          lane_keep_slabs(p, x, 1u, cache);
+        }
       }
     }
     if (__all_sync(0xFFFFFFFFu, got)) break;
@@ -691,11 +727,6 @@ MT_DEV void lane_log_erase(const tree_view& tv, const lane_place& at, const uint
   }
 }
 
-struct defer_list {
-  uint32_t* list;   // requests handed to the tile kernel
-  uint32_t* count;
-};
-
 // Serve the requests of src, one per lane and round (OP_FIND with CONC false:
 // finds that run beside no writer):
 //   1. the lane walks to its border node without locks (lane_locate);
@@ -709,19 +740,27 @@ struct defer_list {
 //      after one fence for the whole warp release their locks.  A lane holds
 //      its locks only inside one round of this loop and never waits for one, so
 //      lanes cannot block each other.
-//   4. A full border node below a parent with room is split in the same way.
-// What does not fit (roots and parents to be split, entries that become new
-// layers, nodes that stay locked) goes to the defer list.
+//      A full border node below a parent with room is split in the same way.
+//   4. What does not fit (roots and parents to be split, entries that become new
+//      layers, nodes that stay locked) is served by the whole warp as one tile,
+//      one request after the other.  Slabs that its lanes took and did not use
+//      are the first that the tile takes.  (A tile kernel after this one, fed
+//      through a list, cost every call a second launch and the latency of the
+//      slowest warp: 1,000 inserts on 100K keys 30 us instead of 26, 2,000 mixed
+//      requests on 200K keys 41 instead of 38, 1M inserts into 1M keys 3.6 ms
+//      instead of 2.9; and what was taken in vain was lost until the next call.
+//      The first large insert after a bulk build, where every node is full, was
+//      faster with it: 200K into 1M keys of 1-8 slices 174 us, now 225.)
 // Measured against tiles of 8 lanes per find and 32 per write: a pair of 1M
 // mixed batches on 16M keys 1.18 ms (4.94), insert + update + find + erase of
-// 300K keys each on 4M keys 0.45 ms (1.57), 1M finds (half of them misses) on 1M
-// keys of 1-8 slices 120 us (357; 70 warp instructions per find instead of 587).
+// 300K keys each on 4M keys 0.46 ms (1.57), 1M finds (half of them misses) on 1M
+// keys of 1-8 slices 124 us (357; 70 warp instructions per find instead of 587).
 // Finds are bound by the load path (64% busy: every node goes through shared
 // memory as one line) and by issue (51%); mixed batches by the latency of up to
 // 17 dependent node visits and two fences per round, with about 4 warps per
 // scheduler: at 3, 4, 5 and 6 blocks per SM they differ by less than 4%.
 template <int OP, bool CONC, class Src>
-MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl) {
+MT_DEV void lane_serve(const tree_view& tv, const Src& src) {
   constexpr uint32_t kAll = 0xFFFFFFFFu;
   constexpr bool kFinds = OP == OP_MIXED || OP == OP_FIND;
   constexpr bool kInserts = OP == OP_MIXED || OP == OP_INSERT || OP == OP_UPSERT;
@@ -733,7 +772,8 @@ MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl
   const pool_view& p = tv.pool;
   const uint32_t n = src.size(), maxV = src.max_value_length();
   const uint32_t per = max(1u, min(32u, (n + warps - 1u) / warps));
-  uint32_t shard = (warp * 0x9E3779B1u) % p.num_shards;
+  slab_cache<32> cache;
+  cache.init(p, warp);
 #pragma unroll 1
   for (uint32_t base = warp * per; base < n; base += warps * per) {
     if (__any_sync(kAll, slot == 0u && fatal_error(p))) break;
@@ -761,7 +801,7 @@ MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl
     // 1. To the border node.
     lane_place at;
     at.idx = 0;
-    at.full = false;
+    at.full = at.stuck = false;
     lane_locate<CONC>(tv, go, key, klen, at);
     bool chain = go && at.found && (at.state == KS_SUFFIX || (find && at.state == KS_LONGVAL));
     if (chain && !p.valid(at.val)) {
@@ -793,6 +833,8 @@ MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl
         if (OP == OP_UPSERT) job = JOB_SET;
       } else if (at.found) {
         defer = true;  // a chain of another key: both move to a new layer
+      } else if (at.stuck) {
+        defer = true;
       } else {
         job = JOB_ADD;
       }
@@ -807,7 +849,7 @@ MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl
         else need = suf_nodes(rest, vlen);
       }
       lane_slabs sl{};
-      if (!warp_take_slabs(p, need + (right_half ? 1u : 0u), shard, sl)) {
+      if (!warp_take_slabs(p, need + (right_half ? 1u : 0u), cache, sl)) {
         job = JOB_NONE;
         defer = true;
         need = 0;
@@ -957,25 +999,34 @@ MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl
       }
     }
     // Chains replaced or erased, and slabs taken in vain.
-    if (kChains && (ns & KS_SLAB) && nv != kInvalid) old_chain = nv;
     if (kWrites && old_chain != kInvalid) lane_retire_chain(p, old_chain);
-    if (kInserts && spare != kInvalid) retire_slab(p, spare);
+    if (kChains && (ns & KS_SLAB) && nv != kInvalid) lane_keep_slabs(p, nv, suf_nodes(rest, vlen), cache);
+    if (kInserts && spare != kInvalid) lane_keep_slabs(p, spare, 1u, cache);
 
-    // 4. Results, and the requests left to the tile kernel.
+    // 4. What is left, by the whole warp as one tile, one request after the other.
     if (kWrites) {
-      const uint32_t dm = __ballot_sync(kAll, defer);
-      if (dm) {
-        uint32_t at0 = 0;
-        if (lane_id() == 0u) at0 = atomicAdd(dl.count, (uint32_t)__popc(dm));
-        at0 = __shfl_sync(kAll, at0, 0);
-        if (defer) dl.list[at0 + __popc(dm & ((1u << lane_id()) - 1u))] = r.id;
+      uint32_t left = __ballot_sync(kAll, defer);
+      const tile<32> t;
+#pragma unroll 1
+      while (left) {
+        const int l = __ffs(left) - 1;
+        left &= left - 1u;
+        const uint32_t* k = reinterpret_cast<const uint32_t*>(t.shfl64(reinterpret_cast<uint64_t>(key), l));
+        const uint32_t* v = reinterpret_cast<const uint32_t*>(t.shfl64(reinterpret_cast<uint64_t>(val), l));
+        const uint32_t kl = t.shfl(klen, l), vl = t.shfl(vlen, l), kind = t.shfl(r.kind, l);
+        int done = RES_FAIL;
+        if (kInserts && kind == MT_REQ_INSERT) done = coop_insert<32, OP == OP_UPSERT>(t, tv, cache, k, kl, v, vl);
+        else if (kUpdates && kind == MT_REQ_UPDATE) done = coop_update<32>(t, tv, cache, k, kl, v, vl);
+        else if (kErases && kind == MT_REQ_ERASE) done = coop_erase<32>(t, tv, k, kl);
+        if ((int)t.rank == l) res = done == RES_OK;
       }
     }
-    if (have != LANE_SKIP && !defer) {
+    if (have != LANE_SKIP) {
       if (kFinds && r.kind == MT_REQ_FIND) src.found(pos, r, present, found_len);
       else src.result(pos, r, res != 0u);
     }
   }
+  if (kWrites) cache.release(tile<32>(), p);
 }
 
 }  // namespace mtb

@@ -30,6 +30,7 @@ namespace mtb {
 
 constexpr uint32_t kInvalid = 0xFFFFFFFFu;
 constexpr int kCtrStride = 32;  // ints: one 128-byte line per counter
+constexpr int kNextWord = 31;   // word of a slab that links a list of slabs
 
 enum mt_err_code : uint32_t {
   ERR_NONE = 0,
@@ -83,6 +84,10 @@ struct slab_cache {
   uint32_t slab = kInvalid;
   uint32_t count = 0;   // uniform over the tile
   uint32_t shard = 0;   // uniform: preferred shard
+  // Whole-warp tiles: slabs that a lane took and led nobody to, a list linked
+  // by their last words (mt_lane.cuh).  They are handed out first.
+  uint32_t vain = kInvalid;
+  uint32_t vain_n = 0;
 
   MT_DEV void init(const pool_view& p, uint32_t tile_id) {
     slab = kInvalid;
@@ -135,6 +140,19 @@ struct slab_cache {
 
   // Returns a fresh slab index (uniform) or kInvalid after recording MT_ERR_OOM.
   MT_DEV uint32_t allocate(const tile<T>& t, const pool_view& p) {
+    if constexpr (T == 32) {
+      const uint32_t m = t.ballot(vain_n != 0u);
+      if (m) {
+        const int l = __ffs(m) - 1;
+        const uint32_t s = t.shfl(vain, l);
+        if ((int)t.rank == l) {
+          vain = ld_relaxed_u32(p.addr(s) + kNextWord);
+          --vain_n;
+        }
+        t.sync();  // the link is read before anyone writes the slab
+        return s;
+      }
+    }
     if (count == 0) {
       for (uint32_t k = 0; k < p.num_shards && count == 0; ++k) {
         const uint32_t s = (shard + k) % p.num_shards;
@@ -168,6 +186,13 @@ MT_DEV void slab_cache<T>::release(const tile<T>& t, const pool_view& p) {
   if (t.rank < count && slab != kInvalid) retire_slab(p, slab);
   count = 0;
   slab = kInvalid;
+  if constexpr (T == 32) {
+    for (; vain_n != 0u; --vain_n) {
+      const uint32_t nx = ld_relaxed_u32(p.addr(vain) + kNextWord);
+      retire_slab(p, vain);
+      vain = nx;
+    }
+  }
 }
 
 }  // namespace mtb

@@ -201,7 +201,7 @@ class GpuMasstree:
     def mixed_batches(self, descriptors, num_subbatches, max_key_length, max_value_length, stream=0,
                       bucket_keys=False, persistent=False, group_by_key=False):
         """Serve num_subbatches mixed batches in order (one request per lane, a
-        kernel pair per sub-batch, or one persistent launch for all with
+        kernel per sub-batch, or one persistent launch for all with
         persistent=True, or all at once with the requests on each key resolved
         in sub-batch order with group_by_key=True).  `descriptors` is a device
         tensor holding mt_subbatch records (see pack_subbatches)."""

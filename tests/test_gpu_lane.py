@@ -161,3 +161,103 @@ def test_updates_of_one_key_in_one_call(n, mixed):
             g.update(keys, two, np.zeros((held, 1), np.uint32), one)
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("form", ["insert", "upsert", "mixed", "batches", "grouped"])
+@pytest.mark.parametrize("held,n", [(1, 3000), (14, 20000), (100, 80000), (3000, 150000)])
+def test_one_call_grows_a_small_tree(form, held, n):
+    # Nearly every insert needs a root or a full parent split, or a new layer
+    # (keys in a few shared prefixes), and the nodes that lanes read first are
+    # split again and again by other warps of the launch.
+    rng = np.random.default_rng(held)
+    keys = np.zeros((held + n, 5), np.uint32)
+    keys[:, 0] = rng.integers(0, 3, held + n)
+    keys[:, 1] = rng.permutation(held + n)
+    keys[:, 2:] = rng.integers(0, 4, (held + n, 3))
+    kl = rng.integers(2, 6, held + n).astype(np.uint32)
+    keys[np.arange(5)[None, :] >= kl[:, None]] = 0
+    vals, vl = np.arange(1, held + n + 1, dtype=np.uint32)[:, None], np.ones(held + n, np.uint32)
+    g, o = GpuIndex(pool_bytes=256 << 20), OracleIndex()
+    try:
+        for x in (g, o):
+            assert x.insert(keys[:held], kl[:held], vals[:held], vl[:held]).all()
+        k, l, v, w = keys[held:], kl[held:], vals[held:], vl[held:]
+        if form in ("insert", "upsert"):
+            res = g.insert(k, l, v, w, upsert=form == "upsert")
+        elif form == "mixed":
+            res = g.mixed(np.zeros(n, np.uint8), k, l, v, w)[2]
+        else:
+            import torch
+            from indexingpu_b200.masstree import pack_subbatches
+            d = [torch.from_numpy(x).cuda() for x in (np.zeros(n, np.uint8), k, l, v, w)]
+            out = torch.zeros(n, dtype=torch.bool, device="cuda")
+            subs = [dict(zip(("types", "keys", "lens", "vals", "vlens", "results", "n"),
+                             [x[p] for x in d] + [out[p], p.stop - p.start])) for p in (slice(0, n // 3), slice(n // 3, n))]
+            g.t.reserve_batches(2, n)
+            g.t.mixed_batches(torch.from_numpy(pack_subbatches(subs)).cuda(), 2, 5, 1, group_by_key=form == "grouped")
+            g.t.sync()
+            res = out.cpu().numpy()
+        assert np.array(res).all() and o.insert(k, l, v, w).all()
+        _same_contents(g, o, held + n, 5, 1)
+    finally:
+        g.close()
+
+
+def test_one_call_of_ascending_keys():
+    # More leaves come off one node during the launch than a walk may visit.
+    n = 1200000
+    g = GpuIndex(pool_bytes=256 << 20)
+    try:
+        keys = np.arange(n + 40, dtype=np.uint32)[:, None]
+        one = np.ones(n + 40, np.uint32)
+        assert g.insert(keys[:40], one[:40], keys[:40], one[:40]).all()
+        assert g.insert(keys[40:], one[40:], keys[40:], one[40:]).all()
+        got, gl = g.find(keys, one, 1)
+        assert (gl == 1).all() and (got == keys).all()
+        ok, count, msg = g.t.validate()
+        assert ok and count == n + 40, msg
+    finally:
+        g.close()
+
+
+def test_slabs_of_inserts_that_lanes_cannot_place():
+    # 1,500 chains of 21 slabs fill half of a pool of 61K slabs.  Into a tree of
+    # 14 keys, lanes place few of them; what they took for the others has to
+    # serve these in the same call.
+    n, maxV = 1500, 620
+    g, o = GpuIndex(pool_bytes=8 << 20), OracleIndex()
+    try:
+        rng = np.random.default_rng(5)
+        keys = rng.permutation(1 << 20)[:n + 14].astype(np.uint32)[:, None]
+        vals = rng.integers(0, 1 << 32, (n + 14, maxV), dtype=np.uint64).astype(np.uint32)
+        one, vl = np.ones(n + 14, np.uint32), np.full(n + 14, maxV, np.uint32)
+        for x in (g, o):
+            assert x.insert(keys[:14], one[:14], vals[:14], vl[:14]).all()
+            assert x.insert(keys[14:], one[14:], vals[14:], vl[14:]).all()
+        _same_contents(g, o, n + 14, 1, maxV)
+    finally:
+        g.close()
+
+
+def test_a_chain_longer_than_a_shard():
+    # A pool of 64 shards of 961 slabs; a value of 30,000 slices takes 1,000.
+    maxV = 30000
+    g, o = GpuIndex(pool_bytes=8 << 20), OracleIndex()
+    try:
+        rng = np.random.default_rng(6)
+        keys = np.arange(20, dtype=np.uint32)[:, None]
+        one = np.ones(20, np.uint32)
+        short = np.full(20, 1, np.uint32)
+        long = np.where(np.arange(20) % 5 == 0, maxV, 40).astype(np.uint32)
+        for vl in (short, long, long):
+            vals = rng.integers(0, 1 << 32, (20, maxV), dtype=np.uint64).astype(np.uint32)
+            vals[np.arange(maxV)[None, :] >= vl[:, None]] = 0
+            for x in (g, o):
+                assert (x.insert if vl is short else x.update)(keys, one, vals, vl).all()
+            _same_contents(g, o, 20, 1, maxV)
+        more = keys + np.uint32(100)
+        for x in (g, o):
+            assert x.insert(more, one, vals, long).all()
+        _same_contents(g, o, 40, 1, maxV)
+    finally:
+        g.close()
