@@ -127,6 +127,51 @@ def test_writes_that_meet_in_one_node(upsert):
         g.close()
 
 
+@pytest.mark.parametrize("n", [1, 5, 37, 400])
+@pytest.mark.parametrize("maxK,maxV", [(150, 80), (92, 1), (2, 121)])
+def test_plain_calls_on_chains_of_many_slabs(n, maxK, maxV):
+    # Warps with one request and with 32; key rests and values that end beside
+    # slab edges; keys that differ from a held one in their last slice only.
+    rng = np.random.default_rng(n + maxK)
+    ends = [e for e in (1, 2, 3, 31, 32, 33, 61, 62, 63, 64, 91, 92, 93, 121, 122, 149, 150) if e <= maxK]
+    vends = [e for e in (1, 2, 29, 30, 31, 59, 60, 61, 80, 90, 119, 120, 121) if e <= maxV]
+    kl, vl = rng.choice(ends, n).astype(np.uint32), rng.choice(vends, n).astype(np.uint32)
+    keys = rng.integers(0, 1 << 32, (n, maxK), dtype=np.uint64).astype(np.uint32)
+    keys[:, 0] = np.arange(n) // 3
+    keys[np.arange(maxK)[None, :] >= kl[:, None]] = 0
+    near = keys.copy()
+    near[np.arange(n), kl - 1] ^= 1
+    keys, kl, vl = np.concatenate([keys, near]), np.concatenate([kl, kl]), np.concatenate([vl, vl[::-1]])
+    _, first = np.unique(np.concatenate([keys, kl[:, None]], axis=1), axis=0, return_index=True)
+    keys, kl, vl = keys[first], kl[first], vl[first]
+    m = len(kl)
+    g, o = GpuIndex(pool_bytes=128 << 20), OracleIndex()
+
+    def values():
+        v = rng.integers(1, 1 << 32, (m, maxV), dtype=np.uint64).astype(np.uint32)
+        l = rng.permutation(vl)
+        v[np.arange(maxV)[None, :] >= l[:, None]] = 0
+        return v, l
+
+    try:
+        half, some = rng.permutation(m)[:(m + 1) // 2], rng.permutation(m)[:(m + 1) // 2]
+        v, l = values()
+        np.testing.assert_array_equal(g.insert(keys[half], kl[half], v[half], l[half]),
+                                      o.insert(keys[half], kl[half], v[half], l[half]))
+        for upsert in (False, True):
+            v, l = values()
+            np.testing.assert_array_equal(g.update(keys, kl, v, l), o.update(keys, kl, v, l))
+            np.testing.assert_array_equal(g.erase(keys[some], kl[some]), o.erase(keys[some], kl[some]))
+            for maxv in (maxV, 1):
+                for x, y in zip(g.find(keys, kl, maxv), o.find(keys, kl, maxv)):
+                    np.testing.assert_array_equal(x, y)
+            v, l = values()
+            np.testing.assert_array_equal(g.insert(keys, kl, v, l, upsert=upsert), o.insert(keys, kl, v, l, upsert=upsert))
+            _same_contents(g, o, m, maxK, maxV)
+    finally:
+        g.close()
+
+
 @pytest.mark.parametrize("n", [2, 255, 256, 257, 1025, 303104, 303105, 310000])
 @pytest.mark.parametrize("mixed", [False, True])
 def test_updates_of_one_key_in_one_call(n, mixed):
