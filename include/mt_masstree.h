@@ -254,6 +254,11 @@ int mt_mixed_batches(mt_masstree* tree, const mt_subbatch* subbatches, uint32_t 
  * library. */
 int mt_set_group_hash_bits(mt_masstree* tree, uint32_t bits);
 
+/* Set the number of the last call that combined updates (a 32-bit count of the
+ * update and mixed-batch calls, after whose last value the combining table is
+ * cleared; for tests of that turn).  New in this library. */
+int mt_set_combine_epoch(mt_masstree* tree, uint32_t epoch);
+
 /* Serving (mt_serve). */
 #define MT_SERVE_SERVED 0u /* device-resident request loop with continuous admission */
 #define MT_SERVE_PLAIN 1u  /* one synchronous mt_mixed_batch call per request, in arrival order */

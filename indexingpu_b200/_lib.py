@@ -46,6 +46,7 @@ SIGNATURES = {
     "mt_server_stop": (_int, [_p]),
     "mt_server_stats": (_int, [_p, _p]),
     "mt_set_group_hash_bits": (_int, [_p, _u32]),
+    "mt_set_combine_epoch": (_int, [_p, _u32]),
 }
 
 

@@ -66,8 +66,9 @@ __global__ void partition_kernel(const uint8_t* types, uint32_t n, uint32_t* fin
 // them, and combine_results_kernel copies the leader's result.
 //
 // The table is never cleared between calls: an entry is (epoch << 32 | request),
-// and the epoch, a device word that every call's reclaim pass moves (so that
-// replayed graphs move it too), makes the entries of earlier calls free.  A block
+// and the epoch, a device word that the reclaim pass of every combining call
+// moves (so that replayed graphs move it too), makes the entries of earlier calls
+// free.  When it comes round, that pass clears the table.  A block
 // first gathers its updates, then works on them with every lane: in a mixed
 // batch with a tenth of updates a warp's three updates otherwise waited for
 // their key rows while the other lanes idled.
@@ -262,10 +263,17 @@ __global__ void line_atomicity_kernel(uint32_t* lines, uint32_t nlines, uint32_t
   }
 }
 
-// Return slabs retired by earlier launches to their shard's free stack; start
-// the call's epoch.
-__global__ void reclaim_kernel(pool_view p, uint32_t* epoch) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) *epoch += 1u;
+// Return slabs retired by earlier launches to their shard's free stack.  Before
+// a combining call (table not null): move the epoch.  Epoch 0 is that of entries
+// never written, so after 2^32 - 1 the table is cleared and 1 follows.
+__global__ void reclaim_kernel(pool_view p, uint32_t* epoch, unsigned long long* table, uint32_t slots) {
+  if (table != nullptr && blockIdx.x == 0) {
+    const uint32_t last = *epoch;
+    __syncthreads();
+    if (last == 0xFFFFFFFFu)
+      for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) table[i] = 0u;
+    if (threadIdx.x == 0) *epoch = last == 0xFFFFFFFFu ? 1u : last + 1u;
+  }
   for (uint32_t s = blockIdx.x; s < p.num_shards; s += gridDim.x) {
     __shared__ int top, n;
     if (threadIdx.x == 0) {
@@ -299,7 +307,7 @@ int host_max_blocks_per_sm(const void* fn, int block, size_t smem) {
   return b;
 }
 int host_launch_reclaim(mt_masstree* t, cudaStream_t s) {
-  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->epoch);
+  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, nullptr, nullptr, 0u);
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
 }
 }  // namespace mtb
@@ -352,10 +360,7 @@ namespace {
 
 int cuda_status(cudaError_t e) { return e == cudaSuccess ? MT_OK : MT_ERR_CUDA; }
 
-int launch_reclaim(mt_masstree* t, cudaStream_t s) {
-  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->epoch);
-  return cuda_status(cudaGetLastError());
-}
+int launch_reclaim(mt_masstree* t, cudaStream_t s) { return host_launch_reclaim(t, s); }
 
 template <int T, int OP, bool CONC>
 int launch_batch_t(mt_masstree* t, const batch_args& a, cudaStream_t s) {
@@ -428,11 +433,12 @@ int ensure_combine_scratch(mt_masstree* t, uint32_t n, cudaStream_t s) {
   return cuda_status(cudaMemsetAsync(t->combine_mem, 0, table, s));
 }
 
-// Combine the updates among the requests of `a` on stream s (after the call's
-// reclaim pass) and set a.leader_of for the kernels that follow.
+// The reclaim pass; then combine the updates among the requests of `a` on stream
+// s and set a.leader_of for the kernels that follow.
 int launch_combine(mt_masstree* t, batch_args& a, cudaStream_t s) {
   const uint32_t slots = combine_slots(t->combine_cap);
   auto* table = reinterpret_cast<unsigned long long*>(t->combine_mem);
+  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->epoch, table, slots);
   uint32_t* leader_of = reinterpret_cast<uint32_t*>(table + slots);
   const uint32_t mask = combine_slots(a.n) - 1u;  // a small call stays within a small part of the table
   const uint32_t chunk = a.n <= (uint32_t)t->sms * 8u * kCombineThreads ? kCombineThreads : kCombineChunk;
@@ -454,7 +460,6 @@ int launch_combine_results(mt_masstree* t, const batch_args& a, uint32_t n, cuda
 int launch_mixed(mt_masstree* t, batch_args a, cudaStream_t s) {
   if (a.n == 0) return MT_OK;
   int rc = ensure_combine_scratch(t, a.n, s);
-  if (!rc) rc = launch_reclaim(t, s);
   if (!rc) rc = launch_combine(t, a, s);
   if (!rc) rc = launch_lane<OP_MIXED>(t, a, s);
   if (!rc) rc = launch_combine_results(t, a, a.n, s);
@@ -684,7 +689,6 @@ int mt_update(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_
   const cudaStream_t s = (cudaStream_t)stream;
   if (n < 2) return launch_writes<OP_UPDATE>(t, a, s);
   int rc = ensure_combine_scratch(t, n, s);
-  if (!rc) rc = launch_reclaim(t, s);
   if (!rc) rc = launch_combine(t, a, s);
   if (!rc) rc = launch_lane<OP_UPDATE>(t, a, s);
   if (!rc) rc = launch_combine_results(t, a, n, s);
@@ -701,6 +705,12 @@ int mt_erase(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_t
   const int rc = host_merge_begin(t, s, flags);
   if (rc) return rc;
   return host_merge_end(t, s, launch_writes<OP_ERASE>(t, a, s));
+}
+
+int mt_set_combine_epoch(mt_masstree* t, uint32_t epoch) {
+  if (!t) return MT_ERR_INVALID_ARG;
+  if (cudaDeviceSynchronize() != cudaSuccess) return MT_ERR_CUDA;
+  return cuda_status(cudaMemcpy(t->epoch, &epoch, sizeof(epoch), cudaMemcpyHostToDevice));
 }
 
 int mt_mixed_batch(mt_masstree* t, const uint8_t* types, const uint32_t* keys, uint32_t maxK,

@@ -306,3 +306,31 @@ def test_a_chain_longer_than_a_shard():
         _same_contents(g, o, 40, 1, maxV)
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("last", [0xFFFFFFFD, 0xFFFFFFFE, 0xFFFFFFFF])
+def test_combining_when_its_count_comes_round(last):
+    # Request 0 is a find of the key that the others update: taken for their
+    # leader (entries never written read as request 0 of call 0), it would keep
+    # them from running.  The entries of the tree's own calls 1 and 2, of more
+    # requests than the later ones, must be gone as well.
+    g = GpuIndex(pool_bytes=64 << 20)
+    try:
+        held = 4000
+        keys, one = np.arange(held, dtype=np.uint32)[:, None], np.ones(held, np.uint32)
+        assert g.insert(keys, one, keys, one).all()
+        for _ in range(2):
+            assert g.update(keys, one, keys + 1, one).all()
+        assert g.t._lib.mt_set_combine_epoch(g.t._h, last) == 0
+        for call in range(4):
+            n = 300
+            ids = np.concatenate([[call], np.full(9, call), np.arange(10, n)]).astype(np.uint32)
+            types = np.full(n, 3, np.uint8)
+            types[0] = 2
+            vals = (ids + np.uint32(1000 * (call + 1)))[:, None]
+            res = np.array(g.mixed(types, ids[:, None], np.ones(n, np.uint32), vals, np.ones(n, np.uint32))[2])
+            assert res[1:].all()
+            got, gl = g.find(keys, one, 1)
+            assert (gl == 1).all() and (got[ids, 0] == vals[:, 0]).all()
+    finally:
+        g.close()
