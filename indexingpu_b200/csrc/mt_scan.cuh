@@ -6,19 +6,22 @@
 // lane reads its own entry's chain line and writes its own output row.  (With
 // one entry after the other, as coop_scan does, a query waits for 13 chain
 // lines per node in turn.)  400K queries of 100 results on 32M keys: 2.01 ms,
-// from 5.25 ms with one entry after the other on 4 lanes (2.30 before the bulk
-// build laid neighbours' chains side by side); bound by random 128-byte lines,
-// of which a result uses a few words.  At 8 blocks per SM; 6 take 2.54 and 10
-// take 2.77 ms, and asking L2 for the next node's chains changes nothing.
+// from 5.25 ms with one entry after the other on 4 lanes; bound by random
+// 128-byte lines, of which a result uses a few words.  (Before the bulk build
+// laid neighbours' chains side by side: 2.30 ms at 8 blocks per SM, 2.54 at 6 and
+// 2.77 at 10, and no change from asking L2 for the next node's chains.  Asking
+// for child layers' roots ahead: 30K bounded scans over layers 124 -> 141 us.)
 #pragma once
 #include "mt_internal.cuh"
 
 namespace mtb {
 
 // Output rows of up to this many slices (key and value together) are written by
-// one lane each; longer ones by the whole tile, one row after the other.
+// one lane each; longer ones by the whole tile, one row after the other.  30K
+// queries of 20 results with rows of 40 + 30 slices: 290 us by lanes, 377 by the
+// tile; 3K queries of one result with rows of 100 + 60 slices: 45 and 28 us.
 #ifndef MT_SCAN_LANE_ROW
-#define MT_SCAN_LANE_ROW 48
+#define MT_SCAN_LANE_ROW 96
 #endif
 constexpr uint32_t kScanLaneRow = MT_SCAN_LANE_ROW;
 
@@ -39,6 +42,8 @@ MT_DEV bool scan_emit_node(const tile<16>& t, const pool_view& p, const scan_fra
     mine = mine && e < start + m;
   }
   if ((o.keys ? o.maxK : 0u) + (o.values ? o.maxV : 0u) > kScanLaneRow) {
+    // The chains are read one after the other: all of them asked for first.
+    if (mine && (st & KS_SLAB)) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.addr(v)));
     for (uint32_t k = start; k < start + m; ++k) {
       const uint32_t ks = t.shfl(st, (int)k), kv = t.shfl(v, (int)k), slice = t.shfl(key, (int)k);
       suffix_head<16> h;

@@ -334,3 +334,39 @@ def test_combining_when_its_count_comes_round(last):
             assert (gl == 1).all() and (got[ids, 0] == vals[:, 0]).all()
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("maxK,maxV", [(40, 8), (8, 40), (31, 17), (48, 48), (49, 48), (70, 30)])
+@pytest.mark.parametrize("count", [1, 14, 60])
+def test_scan_rows_around_the_width_of_one_lane(maxK, maxV, count):
+    # Rows of 48, 96 and 97 slices, of keys alone and of values alone; chains that
+    # end at and beside slab edges.
+    import torch
+    keys, kl, vals, vl = _edge_keys(2500, maxK, maxV, maxK + count)
+    rng = np.random.default_rng(count)
+    g, o = GpuIndex(pool_bytes=128 << 20), OracleIndex()
+    try:
+        for x in (g, o):
+            x.insert(keys, kl, vals, vl)
+        pick = rng.integers(0, len(kl), 300)
+        lower, ll = keys[pick], kl[pick].copy()
+        ll[::7] = np.minimum(ll[::7], 2)
+        upper = lower.copy()
+        upper[:, 1] = np.minimum(upper[:, 1].astype(np.int64) + 3, 0xFFFFFFFF).astype(np.uint32)
+        ul = np.minimum(ll + 1, maxK).astype(np.uint32)
+        for up, ulen in ((None, None), (upper, ul)):
+            want = o.scan(lower, ll, count, up, ulen, maxV=maxV)
+            got = g.scan(lower, ll, count, up, ulen, maxV=maxV)
+            for x, y in zip(got, want):
+                np.testing.assert_array_equal(x, y)
+            d = lambda a: None if a is None else torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+            z = lambda *s: torch.zeros(s, dtype=torch.uint32, device="cuda")  # noqa: E731
+            n = len(ll)
+            okeys, oval = z(n, count, maxK), z(n, count, maxV)
+            g.t.scan(d(lower), d(ll), maxK, count, n, d(up), d(ulen), out_keys=okeys)
+            g.t.scan(d(lower), d(ll), maxK, count, n, d(up), d(ulen), values=oval, max_value_length=maxV)
+            g.t.sync()
+            np.testing.assert_array_equal(oval.cpu().numpy(), want[1])
+            np.testing.assert_array_equal(okeys.cpu().numpy(), want[3])
+    finally:
+        g.close()
