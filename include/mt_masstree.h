@@ -118,8 +118,8 @@ int mt_destroy(mt_masstree* tree);
  * request with a tile of lanes (serving loop, MT_FLAG_PERSISTENT,
  * MT_FLAG_SINGLE_PASS and mt_mixed_batch_noalloc's writes), and resident
  * blocks per SM (0 = as many as fit).  The batch calls themselves serve one
- * request per lane, scans 16 lanes per query, whatever the width.  New in this
- * library. */
+ * request per lane, scans 16 lanes per query (4 for many queries of one or two
+ * results), whatever the width.  New in this library. */
 int mt_set_tile_size(mt_masstree* tree, uint32_t tile_size);
 /* Lanes per request for inserts, updates and erases only (mt_set_tile_size
  * sets both widths). */
@@ -130,8 +130,8 @@ int mt_set_blocks_per_sm(mt_masstree* tree, uint32_t blocks_per_sm);
  * request per lane.  New in this library. */
 int mt_set_upderase_tile_size(mt_masstree* tree, uint32_t tile_size);
 /* Lanes per scan query (4/8/16/32; 0 = the find width, the default).  Accepted
- * and kept; scans use 16 lanes, one per entry of the border node at hand.  New
- * in this library. */
+ * and kept; scans use 16 lanes, one per entry of the border node at hand, or 4
+ * where many queries ask for one or two results.  New in this library. */
 int mt_set_scan_tile_size(mt_masstree* tree, uint32_t tile_size);
 
 /* Bound of every node-lock wait: lock attempts (each followed by a backoff of

@@ -171,9 +171,10 @@ __global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) lane_kernel(tree
   lane_serve<OP, true>(tv, batch_source{a});
 }
 
-template <bool CONC>
+// T 16: a border node's entries side by side (mt_scan.cuh); T 4: one entry after
+// the other, with four times as many queries under way.
+template <int T, bool CONC>
 __global__ void __launch_bounds__(kBlock, MT_SCAN_BLOCKS) scan_kernel(tree_view tv, scan_args a) {
-  constexpr int T = 16;
   tile<T> t;
   const uint32_t tile_id = (blockIdx.x * blockDim.x + threadIdx.x) / T;
   const uint32_t num_tiles = (gridDim.x * blockDim.x) / T;
@@ -212,9 +213,14 @@ __global__ void __launch_bounds__(kBlock, MT_SCAN_BLOCKS) scan_kernel(tree_view 
       o.maxK = a.max_key_length;
       const uint32_t* lower = a.lower + (size_t)q * a.max_key_length;
       const uint32_t* upper = a.upper ? a.upper + (size_t)q * a.max_key_length : nullptr;
-      const uint32_t c = scan_query<CONC>(t, tv, lower, ll, a.use_upper != 0u && upper != nullptr, upper, ul,
-                                          a.max_count, o, frames);
-      if (frames.cur != kInvalid) frames.release(t, tv.pool);
+      const bool use_upper = a.use_upper != 0u && upper != nullptr;
+      uint32_t c;
+      if constexpr (T == 16) {
+        c = scan_query<CONC>(t, tv, lower, ll, use_upper, upper, ul, a.max_count, o, frames);
+        if (frames.cur != kInvalid) frames.release(t, tv.pool);
+      } else {
+        c = coop_scan<T, CONC>(t, tv, lower, ll, use_upper, upper, ul, a.max_count, o, frames);
+      }
       if (t.rank == r) cnt = c;
     }
     if (valid && a.counts) a.counts[i] = cnt;
@@ -466,12 +472,24 @@ int launch_mixed(mt_masstree* t, batch_args a, cudaStream_t s) {
   return rc;
 }
 
+// Scans of so few results (with an upper key: at most so many) by 4 lanes each
+// when there are more than two waves of 16-lane tiles: one entry of a node or two
+// keep few of 16 lanes busy, and the walk is what a query waits for.  60K queries
+// on 1M keys with four shared slices: 1 result 88 us by 4 lanes and 138 by 16, 2
+// 118 and 146, 3 148 and 146; 20K queries of 1 result 48 and 64, 10K 43 and 45.
+// With an upper key 3 results 132 and 168 (75 and 89 the other way round on keys
+// of 1 to 8 slices), 4 156 and 175 (78 and 108).
+constexpr uint32_t kFewResults = 2, kFewResultsUpper = 3;
+
 template <bool CONC>
 int launch_scan(mt_masstree* t, scan_args a, cudaStream_t s) {
-  const int grid = grid_for(t, (const void*)scan_kernel<CONC>);
-  const size_t tiles = (size_t)grid * kBlock / 16;
+  const int grid16 = grid_for(t, (const void*)scan_kernel<16, CONC>);
+  const int grid4 = grid_for(t, (const void*)scan_kernel<4, CONC>);
+  const bool few = a.max_count <= (a.use_upper ? kFewResultsUpper : kFewResults) &&
+                   a.n > 2u * (uint32_t)grid16 * (uint32_t)(kBlock / 16);
+  const size_t tiles = std::max((size_t)grid16 * kBlock / 16, (size_t)grid4 * kBlock / 4);
   if (tiles > t->frames_tiles) {
-    // Scan frames: grown on demand, kept for later calls.
+    // Scan frames, for either width: made once, kept for later calls.
     cudaStreamSynchronize(s);
     if (t->frames) cudaFree(t->frames);
     t->frames = nullptr;
@@ -480,7 +498,8 @@ int launch_scan(mt_masstree* t, scan_args a, cudaStream_t s) {
     t->frames_tiles = tiles;
   }
   a.frames = t->frames;
-  scan_kernel<CONC><<<grid, kBlock, 0, s>>>(t->tv, a);
+  if (few) scan_kernel<4, CONC><<<grid4, kBlock, 0, s>>>(t->tv, a);
+  else scan_kernel<16, CONC><<<grid16, kBlock, 0, s>>>(t->tv, a);
   return cuda_status(cudaGetLastError());
 }
 

@@ -370,3 +370,27 @@ def test_scan_rows_around_the_width_of_one_lane(maxK, maxV, count):
             np.testing.assert_array_equal(okeys.cpu().numpy(), want[3])
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("n", [18944, 18945, 20011])
+@pytest.mark.parametrize("count", [1, 2, 3, 4])
+def test_many_scans_of_few_results(n, count):
+    keys, kl, vals, vl = _edge_keys(4000, 17, 9, 3)
+    rng = np.random.default_rng(n)
+    g, o = GpuIndex(pool_bytes=64 << 20), OracleIndex()
+    try:
+        for x in (g, o):
+            x.insert(keys, kl, vals, vl)
+        pick = rng.integers(0, len(kl), n)
+        lower, ll = keys[pick], kl[pick]
+        near = np.arange(n) % 3 == 0
+        lower[near, ll[near] - 1] ^= 1
+        upper, ul = lower.copy(), ll.copy()
+        upper[:, 0] = np.minimum(upper[:, 0].astype(np.int64) + np.arange(n) % 2, 0xFFFFFFFF).astype(np.uint32)
+        for up, ulen in ((None, None), (upper, ul)):
+            want = o.scan(lower, ll, count, up, ulen, maxV=9)
+            for conc in (False, True):
+                for x, y in zip(g.scan(lower, ll, count, up, ulen, maxV=9, concurrent=conc), want):
+                    np.testing.assert_array_equal(x, y)
+    finally:
+        g.close()
