@@ -50,11 +50,11 @@ enum { MT_REQ_INSERT = 0, MT_REQ_ERASE = 1, MT_REQ_FIND = 2, MT_REQ_UPDATE = 3 }
 #define MT_FLAG_USE_UPPER_KEY 4u    /* scan stops after upper_keys (reference `use_upper_key`) */
 #define MT_FLAG_SINGLE_PASS 8u      /* mixed_batch: one kernel for every kind instead of
                                        finds-then-writes passes (comparison switch) */
-#define MT_FLAG_BUCKET_KEYS 16u     /* mixed_batches: serve short keys before long keys in
-                                       every request class (accepted by mixed_batch, which
-                                       serves its requests without classes) */
+#define MT_FLAG_BUCKET_KEYS 16u     /* mixed_batches with MT_FLAG_PERSISTENT: serve short keys
+                                       before long keys in every request class (accepted by the
+                                       other forms and mixed_batch, which have no classes) */
 #define MT_FLAG_PERSISTENT 32u      /* mixed_batches: one cooperative persistent launch for all
-                                       sub-batches instead of a kernel pair per sub-batch */
+                                       sub-batches instead of a kernel per sub-batch */
 #define MT_FLAG_MERGE 64u           /* erase, mixed_batch: after the call's erases, fold nodes
                                        left with 4 entries or fewer into a neighbour under the same
                                        parent, border nodes and then their sparse ancestors, and
@@ -105,8 +105,8 @@ typedef struct mt_stats_t {
 
 /* Construction.  Replaces gpu_masstree(allocator(pool_ratio), reclaimer())
  * (reference gpu_masstree.hpp:67-72, simple_slab_alloc.hpp:56-69): the slab
- * pool takes pool_ratio of the currently free device memory (a few KB of
- * counters are allocated beside it).
+ * pool takes pool_ratio of the currently free device memory (a little is
+ * allocated beside it: counters and a list of at most 1/256 of the pool).
  * tile_size: see mt_set_tile_size. */
 int mt_create(mt_masstree** out, float pool_ratio, uint32_t tile_size);
 /* Same, with the pool size given in bytes. */
@@ -116,7 +116,8 @@ int mt_destroy(mt_masstree* tree);
 
 /* Launch shape: lanes per request (4/8/16/32) of the kernels that serve a
  * request with a tile of lanes (serving loop, MT_FLAG_PERSISTENT,
- * MT_FLAG_SINGLE_PASS and mt_mixed_batch_noalloc's writes), and resident
+ * MT_FLAG_SINGLE_PASS, mt_mixed_batch_noalloc's writes, and the requests that
+ * the one-request-per-lane kernels of large calls hand on), and resident
  * blocks per SM (0 = as many as fit).  The batch calls themselves serve one
  * request per lane, scans 16 lanes per query (4 for many queries of one or two
  * results), whatever the width.  New in this library. */

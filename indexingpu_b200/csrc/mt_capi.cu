@@ -82,10 +82,11 @@ MT_DEV uint64_t key_hash(const uint32_t* k, uint32_t klen) {
   return h ^ (h >> 29);
 }
 
-// Requests that a block looks at together: 1,024, or as many as it has threads
-// while that leaves no block of the launch a second chunk.  (In chunks of 1,024
-// a call of 1,000 updates with 150-slice keys, all of them hashed and compared
-// by one block, took 124 us and takes 82; 20,000 of them 206 and 118.)
+// Requests that a block looks at together: 1,024, or fewer (down to as many as it
+// has threads) while that leaves SMs with less than two blocks.  (In chunks of
+// 1,024 a call of 1,000 updates with 150-slice keys, all of them hashed and
+// compared by one block, took 124 us and takes 82; 20,000 of them 206 and 118.
+// In chunks of 256, 300,000 updates of 8-slice keys took 128 us instead of 124.)
 constexpr uint32_t kCombineThreads = 256, kCombineChunk = 1024;
 __global__ void __launch_bounds__(kCombineThreads) combine_kernel(batch_args a, unsigned long long* table,
                                                                   uint32_t mask, uint32_t* leader_of,
@@ -155,6 +156,7 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for<OP>) batch_kernel(tree_
   const uint32_t num_tiles = (gridDim.x * blockDim.x) / T;
   slab_cache<T> cache;
   cache.init(tv.pool, tile_id);
+  cache.last_resort = true;
   serve_requests<T, OP, CONC>(t, tv, cache, a, tile_id, num_tiles);
   cache.release(t, tv.pool);
 }
@@ -166,9 +168,9 @@ __global__ void __launch_bounds__(kBlock, MT_LANE_FIND_BLOCKS) find_kernel(tree_
 
 // Inserts, updates, erases and mixed batches, one request per lane (what bounds
 // them and what they measured: lane_serve).
-template <int OP>
-__global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) lane_kernel(tree_view tv, batch_args a) {
-  lane_serve<OP, true>(tv, batch_source{a});
+template <int OP, bool TAIL>
+__global__ void __launch_bounds__(kBlock, MT_LANE_WRITE_BLOCKS) lane_kernel(tree_view tv, batch_args a, defer_list dl) {
+  lane_serve<OP, true, TAIL>(tv, batch_source{a}, dl);
 }
 
 // T 16: a border node's entries side by side (mt_scan.cuh); T 4: one entry after
@@ -271,8 +273,11 @@ __global__ void line_atomicity_kernel(uint32_t* lines, uint32_t nlines, uint32_t
 
 // Return slabs retired by earlier launches to their shard's free stack.  Before
 // a combining call (table not null): move the epoch.  Epoch 0 is that of entries
-// never written, so after 2^32 - 1 the table is cleared and 1 follows.
-__global__ void reclaim_kernel(pool_view p, uint32_t* epoch, unsigned long long* table, uint32_t slots) {
+// never written, so after 2^32 - 1 the table is cleared and 1 follows.  The call's
+// list of handed requests starts empty.
+__global__ void reclaim_kernel(pool_view p, uint32_t* epoch, unsigned long long* table, uint32_t slots,
+                               uint32_t* handed) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *handed = 0u;
   if (table != nullptr && blockIdx.x == 0) {
     const uint32_t last = *epoch;
     __syncthreads();
@@ -281,23 +286,26 @@ __global__ void reclaim_kernel(pool_view p, uint32_t* epoch, unsigned long long*
     if (threadIdx.x == 0) *epoch = last == 0xFFFFFFFFu ? 1u : last + 1u;
   }
   for (uint32_t s = blockIdx.x; s < p.num_shards; s += gridDim.x) {
-    __shared__ int top, n;
+    __shared__ int top, n, back;
     if (threadIdx.x == 0) {
       top = max(*p.top(s), 0);
       n = *p.limbo_count(s);
-      if (top + n > (int)p.shard_slabs) {
+      back = *p.unused_count(s);
+      if (top + n + back > (int)p.shard_slabs) {
         record_error(p, ERR_CORRUPT, MT_AT(SRC_CAPI));
-        n = 0;
+        n = back = 0;
       }
     }
     __syncthreads();
     uint32_t* stack = p.free_stack + (size_t)s * p.shard_slabs;
     const uint32_t* limbo = p.limbo + (size_t)s * p.shard_slabs;
     for (int i = threadIdx.x; i < n; i += blockDim.x) stack[top + i] = limbo[i];
+    for (int i = threadIdx.x; i < back; i += blockDim.x) stack[top + n + i] = limbo[(int)p.shard_slabs - 1 - i];
     __syncthreads();
     if (threadIdx.x == 0) {
-      *p.top(s) = top + n;
+      *p.top(s) = top + n + back;
       *p.limbo_count(s) = 0;
+      *p.unused_count(s) = 0;
     }
     __syncthreads();
   }
@@ -313,7 +321,7 @@ int host_max_blocks_per_sm(const void* fn, int block, size_t smem) {
   return b;
 }
 int host_launch_reclaim(mt_masstree* t, cudaStream_t s) {
-  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, nullptr, nullptr, 0u);
+  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, nullptr, nullptr, 0u, t->defer_mem);
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_CUDA;
 }
 }  // namespace mtb
@@ -386,18 +394,30 @@ int launch_batch_tile(mt_masstree* t, uint32_t tile, const batch_args& a, cudaSt
   }
 }
 
-// Writes and mixed batches, one request per lane.  The reclaim pass is the
+// Writes and mixed batches, one request per lane; with more requests than lanes
+// (and room for them in the list), those that lanes cannot place by a tile kernel
+// after it (lane_serve says why the line lies there).  The reclaim pass is the
 // caller's.
 template <int OP>
-int launch_lane(mt_masstree* t, const batch_args& a, cudaStream_t s) {
-  lane_kernel<OP><<<host_lane_grid(t, (const void*)lane_kernel<OP>, a.n), kBlock, 0, s>>>(t->tv, a);
-  return cuda_status(cudaGetLastError());
+int launch_lane(mt_masstree* t, const batch_args& a, uint32_t tile, cudaStream_t s) {
+  const int grid = host_lane_grid(t, (const void*)lane_kernel<OP, false>, a.n);
+  if (a.n <= (uint32_t)grid * (uint32_t)kBlock || a.n > t->defer_cap) {
+    lane_kernel<OP, false><<<grid, kBlock, 0, s>>>(t->tv, a, defer_list{});
+    return cuda_status(cudaGetLastError());
+  }
+  const defer_list dl{t->defer_mem + 32, t->defer_mem};
+  lane_kernel<OP, true><<<host_lane_grid(t, (const void*)lane_kernel<OP, true>, a.n), kBlock, 0, s>>>(t->tv, a, dl);
+  if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
+  batch_args d = a;
+  d.index = dl.list;
+  d.n_dev = dl.count;
+  return launch_batch_tile<OP, true>(t, tile, d, s);
 }
 template <int OP>
 int launch_writes(mt_masstree* t, const batch_args& a, cudaStream_t s) {
   if (a.n == 0) return MT_OK;
   const int rc = launch_reclaim(t, s);
-  return rc ? rc : launch_lane<OP>(t, a, s);
+  return rc ? rc : launch_lane<OP>(t, a, t->write_tile_size, s);
 }
 
 // Finds take no slabs, so no reclaim pass precedes them.  a.n: the number of
@@ -444,10 +464,11 @@ int ensure_combine_scratch(mt_masstree* t, uint32_t n, cudaStream_t s) {
 int launch_combine(mt_masstree* t, batch_args& a, cudaStream_t s) {
   const uint32_t slots = combine_slots(t->combine_cap);
   auto* table = reinterpret_cast<unsigned long long*>(t->combine_mem);
-  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->epoch, table, slots);
+  reclaim_kernel<<<kShards, 256, 0, s>>>(t->tv.pool, t->epoch, table, slots, t->defer_mem);
   uint32_t* leader_of = reinterpret_cast<uint32_t*>(table + slots);
   const uint32_t mask = combine_slots(a.n) - 1u;  // a small call stays within a small part of the table
-  const uint32_t chunk = a.n <= (uint32_t)t->sms * 8u * kCombineThreads ? kCombineThreads : kCombineChunk;
+  const uint32_t share = a.n / (2u * (uint32_t)t->sms) / kCombineThreads;  // in full sets of threads
+  const uint32_t chunk = std::min(kCombineChunk, (share + 1u) * kCombineThreads);
   const int grid = std::max(1, std::min<int>(t->sms * 8, (int)(a.n / chunk + (a.n % chunk != 0u))));
   combine_kernel<<<grid, kCombineThreads, 0, s>>>(a, table, mask, leader_of, t->epoch, chunk);
   if (cudaGetLastError() != cudaSuccess) return MT_ERR_CUDA;
@@ -467,7 +488,7 @@ int launch_mixed(mt_masstree* t, batch_args a, cudaStream_t s) {
   if (a.n == 0) return MT_OK;
   int rc = ensure_combine_scratch(t, a.n, s);
   if (!rc) rc = launch_combine(t, a, s);
-  if (!rc) rc = launch_lane<OP_MIXED>(t, a, s);
+  if (!rc) rc = launch_lane<OP_MIXED>(t, a, t->write_tile_size <= 16 ? 16u : 32u, s);
   if (!rc) rc = launch_combine_results(t, a, a.n, s);
   return rc;
 }
@@ -527,8 +548,11 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
   const size_t stack_bytes = nslabs * 4u;
   const size_t ctr_bytes = (size_t)kShards * 3u * kCtrStride * sizeof(int);
   const size_t err_bytes = 128;
-  const size_t epoch_bytes = 128;
-  const size_t total = slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes + epoch_bytes;
+  const size_t epoch_bytes = 128, count_bytes = 128;
+  // The list of handed requests: 1/256 of the pool, at most 16M entries.
+  const uint64_t defer_cap = std::min<uint64_t>(1u << 24, std::max<uint64_t>(4096u, pool_bytes / 1024u));
+  const size_t total =
+      slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes + epoch_bytes + count_bytes + defer_cap * 4u;
   if (cudaMalloc(&t->mem, total) != cudaSuccess) { delete t; return MT_ERR_OOM; }
   char* base = (char*)t->mem;
   pool_view& p = t->tv.pool;
@@ -538,11 +562,13 @@ int create_impl(mt_masstree** out, uint64_t pool_bytes, uint32_t tile_size) {
   p.ctr = (int*)(base + slab_bytes + 2 * stack_bytes);
   p.err = (uint32_t*)(base + slab_bytes + 2 * stack_bytes + ctr_bytes);
   t->epoch = (uint32_t*)(base + slab_bytes + 2 * stack_bytes + ctr_bytes + err_bytes);
+  t->defer_mem = t->epoch + epoch_bytes / 4u;
+  t->defer_cap = (uint32_t)defer_cap;
   p.num_slabs = (uint32_t)nslabs;
   p.num_shards = kShards;
   p.shard_slabs = shard_slabs;
   p.lock_spins = kLockSpins;
-  cudaError_t e = cudaMemset(p.ctr, 0, ctr_bytes + err_bytes + epoch_bytes);
+  cudaError_t e = cudaMemset(p.ctr, 0, ctr_bytes + err_bytes + epoch_bytes + count_bytes);
   // Root of trie layer 0 = slab 0 (shard 0's bump pointer starts past it).
   uint32_t root_img[32] = {0};
   root_img[WORD_HIGH] = 0xFFFFFFFFu;
@@ -709,7 +735,7 @@ int mt_update(mt_masstree* t, const uint32_t* keys, uint32_t maxK, const uint32_
   if (n < 2) return launch_writes<OP_UPDATE>(t, a, s);
   int rc = ensure_combine_scratch(t, n, s);
   if (!rc) rc = launch_combine(t, a, s);
-  if (!rc) rc = launch_lane<OP_UPDATE>(t, a, s);
+  if (!rc) rc = launch_lane<OP_UPDATE>(t, a, t->write_tile_size, s);
   if (!rc) rc = launch_combine_results(t, a, n, s);
   return rc;
 }
@@ -816,7 +842,7 @@ int mt_stats(mt_masstree* t, mt_stats_t* out) {
   for (uint32_t s = 0; s < p.num_shards; ++s) {
     const int top = h[(3 * s + 0) * kCtrStride];
     const int bump = h[(3 * s + 1) * kCtrStride];
-    const int lim = h[(3 * s + 2) * kCtrStride];
+    const int lim = h[(3 * s + 2) * kCtrStride] + h[(3 * s + 2) * kCtrStride + 1];  // retired, and given back unused
     handed += (uint64_t)std::min<int>(std::max(bump, 0), (int)p.shard_slabs);
     stacked += (uint64_t)std::max(top, 0);
     limbo += (uint64_t)std::max(lim, 0);
@@ -1003,6 +1029,11 @@ extern "C" int mt_validate(mt_masstree* t, uint64_t* num_keys, char* msg, size_t
       return MT_ERR_CUDA;
     if (lim > 0 && cudaMemcpy(freed.data() + base + top, p.limbo + (size_t)s * p.shard_slabs, (size_t)lim * 4u,
                               cudaMemcpyDeviceToHost) != cudaSuccess)
+      return MT_ERR_CUDA;
+    const int back = std::max(h[(3 * s + 2) * kCtrStride + 1], 0);
+    freed.resize(base + top + lim + back);
+    if (back > 0 && cudaMemcpy(freed.data() + base + top + lim, p.limbo + (size_t)(s + 1) * p.shard_slabs - back,
+                               (size_t)back * 4u, cudaMemcpyDeviceToHost) != cudaSuccess)
       return MT_ERR_CUDA;
   }
   bool good = v.layer(t->tv.root, 0);

@@ -229,6 +229,8 @@ struct mt_masstree {
   uint32_t* combine_mem = nullptr;  // update-combining scratch (grown on demand)
   uint32_t combine_cap = 0;
   uint32_t* epoch = nullptr;        // number of the call in the combining table (device)
+  uint32_t* defer_mem = nullptr;    // requests that large launches hand on: count (one line), then defer_cap entries
+  uint32_t defer_cap = 0;
   mt_host_pipe* host_pipe = nullptr;
   void* mem = nullptr;
   mtb::tree_view tv{};

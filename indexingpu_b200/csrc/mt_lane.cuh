@@ -440,8 +440,19 @@ MT_DEV uint32_t lane_slab(const pool_view& p, const lane_slabs& s, uint32_t q) {
   return s.shard * p.shard_slabs + s.bump + (k - s.n_stack);
 }
 
-// Keep a chain of n slabs that nothing leads to in the warp's slab cache (one lane).
+// Keep a chain of n slabs that nothing leads to in the warp's slab cache, or
+// (TAIL) give it back for the kernel that follows (one lane).
+template <bool TAIL>
 MT_DEV void lane_keep_slabs(const pool_view& p, uint32_t head, uint32_t n, slab_cache<32>& cache) {
+  if (TAIL) {
+#pragma unroll 1
+    for (uint32_t q = 0; q < n; ++q) {
+      const uint32_t next = q + 1u < n ? ld_relaxed_u32(p.addr(head) + kNextWord) : kInvalid;
+      return_unused(p, head);
+      head = next;
+    }
+    return;
+  }
   uint32_t tail = head;
 #pragma unroll 1
   for (uint32_t q = 1; q < n; ++q) tail = ld_relaxed_u32(p.addr(tail) + kNextWord);
@@ -455,6 +466,7 @@ MT_DEV void lane_keep_slabs(const pool_view& p, uint32_t head, uint32_t n, slab_
 // serves the first lanes; the next shards serve the others.  Returns whether
 // the lane got its slabs (no error is recorded: a tile, which takes one slab
 // after the other from any shard, serves the request then).
+template <bool TAIL>
 MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, slab_cache<32>& cache, lane_slabs& s) {
   const uint32_t lane = lane_id();
   uint32_t& shard = cache.shard;
@@ -511,11 +523,11 @@ MT_DEV bool warp_take_slabs(const pool_view& p, uint32_t need, slab_cache<32>& c
         s = g;
         got = true;
       } else {
-        // The part of a lane's need that this shard covered stays with the warp.
+        // The part of a lane's need that this shard covered is kept, or given back.
 #pragma unroll 1
         for (uint32_t q = g.first; q < have; ++q) {
           const uint32_t x = lane_slab(p, g, q - g.first);
-          lane_keep_slabs(p, x, 1u, cache);
+          lane_keep_slabs<TAIL>(p, x, 1u, cache);
         }
       }
     }
@@ -746,6 +758,13 @@ MT_DEV void lane_log_erase(const tree_view& tv, const lane_place& at, const uint
   }
 }
 
+// Where a launch that is followed by a tile kernel puts the requests that lanes
+// cannot place (room for all of the launch's requests).
+struct defer_list {
+  uint32_t* list;
+  uint32_t* count;
+};
+
 // Serve the requests of src, one per lane and round (OP_FIND with CONC false:
 // finds that run beside no writer):
 //   1. the lane walks to its border node without locks (lane_locate);
@@ -764,12 +783,14 @@ MT_DEV void lane_log_erase(const tree_view& tv, const lane_place& at, const uint
 //      layers, nodes that stay locked) is served by the whole warp as one tile,
 //      one request after the other.  Slabs that its lanes took and did not use
 //      are the first that the tile takes.  (A tile kernel after this one, fed
-//      through a list, cost every call a second launch and the latency of the
+//      through a list, costs a small call a second launch and the latency of the
 //      slowest warp: 1,000 inserts on 100K keys 30 us instead of 26, 2,000 mixed
-//      requests on 200K keys 41 instead of 38, 1M inserts into 1M keys 3.6 ms
-//      instead of 2.9; and what was taken in vain was lost until the next call.
-//      The first large insert after a bulk build, where every node is full, was
-//      faster with it: 200K into 1M keys of 1-8 slices 174 us, now 225.)
+//      requests on 200K keys 41 instead of 38.)
+//      In a launch of more than one round (TAIL), where the other lanes' next
+//      requests would wait, they go to that list and the slabs taken for them are
+//      the last resort of the tile kernel's allocations: a 1M mixed batch with
+//      300K new keys 0.78 ms with warps serving them, 0.61 with the list; 200K
+//      inserts into 1M keys of 1-8 slices 225 and 174 us.
 // Measured against tiles of 8 lanes per find and 32 per write: a pair of 1M
 // mixed batches on 16M keys 1.18 ms (4.94), insert + update + find + erase of
 // 300K keys each on 4M keys 0.46 ms (1.57), 1M finds (half of them misses) on 1M
@@ -778,8 +799,8 @@ MT_DEV void lane_log_erase(const tree_view& tv, const lane_place& at, const uint
 // memory as one line) and by issue (51%); mixed batches by the latency of up to
 // 17 dependent node visits and two fences per round, with about 4 warps per
 // scheduler: at 3, 4, 5 and 6 blocks per SM they differ by less than 4%.
-template <int OP, bool CONC, class Src>
-MT_DEV void lane_serve(const tree_view& tv, const Src& src) {
+template <int OP, bool CONC, bool TAIL = false, class Src>
+MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl = defer_list{}) {
   constexpr uint32_t kAll = 0xFFFFFFFFu;
   constexpr bool kFinds = OP == OP_MIXED || OP == OP_FIND;
   constexpr bool kInserts = OP == OP_MIXED || OP == OP_INSERT || OP == OP_UPSERT;
@@ -868,7 +889,7 @@ MT_DEV void lane_serve(const tree_view& tv, const Src& src) {
         else need = suf_nodes(rest, vlen);
       }
       lane_slabs sl{};
-      if (!warp_take_slabs(p, need + (right_half ? 1u : 0u), cache, sl)) {
+      if (!warp_take_slabs<TAIL>(p, need + (right_half ? 1u : 0u), cache, sl)) {
         job = JOB_NONE;
         defer = true;
         need = 0;
@@ -1019,11 +1040,21 @@ MT_DEV void lane_serve(const tree_view& tv, const Src& src) {
     }
     // Chains replaced or erased, and slabs taken in vain.
     if (kWrites && old_chain != kInvalid) lane_retire_chain(p, old_chain);
-    if (kChains && (ns & KS_SLAB) && nv != kInvalid) lane_keep_slabs(p, nv, suf_nodes(rest, vlen), cache);
-    if (kInserts && spare != kInvalid) lane_keep_slabs(p, spare, 1u, cache);
+    if (kChains && (ns & KS_SLAB) && nv != kInvalid) lane_keep_slabs<TAIL>(p, nv, suf_nodes(rest, vlen), cache);
+    if (kInserts && spare != kInvalid) lane_keep_slabs<TAIL>(p, spare, 1u, cache);
 
-    // 4. What is left, by the whole warp as one tile, one request after the other.
-    if (kWrites) {
+    // 4. What is left: to the list, or by the whole warp as one tile, one request
+    // after the other.
+    if (kWrites && TAIL) {
+      const uint32_t m = __ballot_sync(kAll, defer);
+      if (m) {
+        uint32_t at0 = 0;
+        if (lane_id() == 0u) at0 = atomicAdd(dl.count, (uint32_t)__popc(m));
+        at0 = __shfl_sync(kAll, at0, 0);
+        if (defer) dl.list[at0 + __popc(m & ((1u << lane_id()) - 1u))] = r.id;
+      }
+    }
+    if constexpr (kWrites && !TAIL) {
       uint32_t left = __ballot_sync(kAll, defer);
       const tile<32> t;
 #pragma unroll 1
@@ -1040,12 +1071,12 @@ MT_DEV void lane_serve(const tree_view& tv, const Src& src) {
         if ((int)t.rank == l) res = done == RES_OK;
       }
     }
-    if (have != LANE_SKIP) {
+    if (have != LANE_SKIP && !(TAIL && defer)) {
       if (kFinds && r.kind == MT_REQ_FIND) src.found(pos, r, present, found_len);
       else src.result(pos, r, res != 0u);
     }
   }
-  if (kWrites) cache.release(tile<32>(), p);
+  if (kWrites && !TAIL) cache.release(tile<32>(), p);
 }
 
 }  // namespace mtb

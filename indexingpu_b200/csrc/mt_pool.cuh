@@ -59,6 +59,9 @@ struct pool_view {
   MT_HD int* top(uint32_t s) const { return ctr + (size_t)(3u * s + 0u) * kCtrStride; }
   MT_HD int* bump(uint32_t s) const { return ctr + (size_t)(3u * s + 1u) * kCtrStride; }
   MT_HD int* limbo_count(uint32_t s) const { return ctr + (size_t)(3u * s + 2u) * kCtrStride; }
+  // Slabs given back by a launch that led nobody to them: the other end of the
+  // shard's limbo array (entry i at shard_slabs - 1 - i).
+  MT_HD int* unused_count(uint32_t s) const { return limbo_count(s) + 1; }
 };
 
 // Where an error was detected: a source file number (high 16 bits) and line.
@@ -88,6 +91,9 @@ struct slab_cache {
   // by their last words (mt_lane.cuh).  They are handed out first.
   uint32_t vain = kInvalid;
   uint32_t vain_n = 0;
+  // Set by kernels that follow one that gave slabs back unused: these are taken
+  // when every shard is empty.
+  bool last_resort = false;
 
   MT_DEV void init(const pool_view& p, uint32_t tile_id) {
     slab = kInvalid;
@@ -159,6 +165,27 @@ struct slab_cache {
         count = refill_from(t, p, s);
         if (count) shard = s;
       }
+      if (count == 0 && last_resort) {
+        uint64_t at = 0;
+        if (t.leader()) {
+          for (uint32_t s = 0; s < p.num_shards && count == 0; ++s) {
+            int c = (int)ld_relaxed_u32((const uint32_t*)p.unused_count(s));
+            while (c > 0) {
+              const int n = min(c, T);
+              const int old = atomicCAS(p.unused_count(s), c, c - n);
+              if (old == c) {
+                at = (uint64_t)(s + 1u) * p.shard_slabs - (uint64_t)c;
+                count = (uint32_t)n;
+                break;
+              }
+              c = old;
+            }
+          }
+        }
+        count = t.shfl(count, 0);
+        at = t.shfl64(at, 0);
+        slab = t.rank < count ? ld_relaxed_u32(p.limbo + at + t.rank) : kInvalid;
+      }
       if (count == 0) {
         if (t.leader()) record_error(p, ERR_OOM, MT_AT(SRC_POOL));
         return kInvalid;
@@ -179,6 +206,15 @@ MT_DEV void retire_slab(const pool_view& p, uint32_t slab) {
   const int pos = atomicAdd(p.limbo_count(s), 1);
   if (pos >= (int)p.shard_slabs) { record_error(p, ERR_CORRUPT, MT_AT(SRC_POOL)); return; }
   p.limbo[(size_t)s * p.shard_slabs + pos] = slab;
+}
+
+// Give back a slab that nothing led to (called by one lane).  No reader can hold
+// it, so a launch that gives nothing back itself may hand it out again within the
+// same call (slab_cache::last_resort).
+MT_DEV void return_unused(const pool_view& p, uint32_t slab) {
+  const uint32_t s = slab / p.shard_slabs;
+  const int pos = atomicAdd(p.unused_count(s), 1);
+  p.limbo[(size_t)(s + 1u) * p.shard_slabs - 1u - pos] = slab;
 }
 
 template <int T>

@@ -172,10 +172,10 @@ def test_plain_calls_on_chains_of_many_slabs(n, maxK, maxV):
         g.close()
 
 
-@pytest.mark.parametrize("n", [2, 255, 256, 257, 1025, 303104, 303105, 310000])
+@pytest.mark.parametrize("n", [2, 255, 256, 257, 1025, 75775, 75776, 151553, 227328, 310000])
 @pytest.mark.parametrize("mixed", [False, True])
 def test_updates_of_one_key_in_one_call(n, mixed):
-    # Chunks of 256 and of 1,024 requests per block, whole and ragged; a call
+    # Chunks of 256 to 1,024 requests per block, whole and ragged; a call
     # after smaller and larger ones (the table keeps the entries of earlier
     # calls).  Updates of one key have no order: the result is every request's,
     # the value one of theirs.
@@ -249,9 +249,10 @@ def test_one_call_grows_a_small_tree(form, held, n):
 
 
 def test_one_call_of_ascending_keys():
-    # More leaves come off one node during the launch than a walk may visit.
+    # More leaves come off one node during the launch than a walk may visit, and
+    # more requests are left to tiles than the list for them has room for.
     n = 1200000
-    g = GpuIndex(pool_bytes=256 << 20)
+    g = GpuIndex(pool_bytes=48 << 20)
     try:
         keys = np.arange(n + 40, dtype=np.uint32)[:, None]
         one = np.ones(n + 40, np.uint32)
@@ -265,12 +266,12 @@ def test_one_call_of_ascending_keys():
         g.close()
 
 
-def test_slabs_of_inserts_that_lanes_cannot_place():
-    # 1,500 chains of 21 slabs fill half of a pool of 61K slabs.  Into a tree of
-    # 14 keys, lanes place few of them; what they took for the others has to
-    # serve these in the same call.
-    n, maxV = 1500, 620
-    g, o = GpuIndex(pool_bytes=8 << 20), OracleIndex()
+@pytest.mark.parametrize("n,maxV,pool_mb", [(1500, 620, 8), (90000, 110, 96)])
+def test_slabs_of_inserts_that_lanes_cannot_place(n, maxV, pool_mb):
+    # The chains (of 21 and of 4 slabs) fill half of the pool.  Into a tree of 14
+    # keys, lanes place few of them; what they took for the others has to serve
+    # these in the same call (of the second one: in its second kernel).
+    g, o = GpuIndex(pool_bytes=pool_mb << 20), OracleIndex()
     try:
         rng = np.random.default_rng(5)
         keys = rng.permutation(1 << 20)[:n + 14].astype(np.uint32)[:, None]
