@@ -49,7 +49,7 @@ def parse():
     ap.add_argument("--tile", type=int, default=8, help="lanes per find")
     ap.add_argument("--write-tile", type=int, default=32, help="lanes per insert/update/erase")
     ap.add_argument("--upderase-tile", type=int, default=0,
-                    help="lanes per update/erase of a mixed batch (0: the write width)")
+                    help="accepted and passed on (mixed batches serve one request per lane)")
     ap.add_argument("--scan-tile", type=int, default=4, help="lanes per scan query (c3 section)")
     ap.add_argument("--blocks-per-sm", type=int, default=0)
     ap.add_argument("--bucket", type=int, default=0, help="1: mixed_batch serves short keys before long keys")
@@ -382,9 +382,8 @@ def run_ours(args, rank, world, dist):
                                    "after a 16M-key preload; keys 2-16 slices, 4096 shared prefixes; values 1-8 slices",
                        "preload_keys": args.preload, "batch_requests": args.batch, "max_key_length": MAXK,
                        "max_value_length": MAXV, "tile_size": args.tile, "write_tile_size": args.write_tile,
-                       "upderase_tile_size": args.upderase_tile or args.write_tile,
                        "form": "plain per-call mixed_batch (reclaim, update combining, one request per lane, tile kernel "
-                               "for the rest, results of combined updates)",
+                               "for what lanes hand on, results of combined updates)",
                        "l2": "no flush: the index (>2 GB of slabs) and each batch's inputs exceed the 126 MB L2",
                        "parallelism": f"replicas x{world}"},
             "batch_latency_ms": {"p50": round(sorted_steps[len(sorted_steps) // 2], 4),
@@ -399,12 +398,12 @@ def run_ours(args, rank, world, dist):
                          "frac": round(achieved / peak, 4), "peak_source": peak_kind,
                          "traffic": None if tr is None else int(tr * args.batch),
                          "algorithmic_bytes_per_step": abytes // args.steps,
-                         "kernel": "mixed_batch call: reclaim + combining + lane kernel + rest"},
+                         "kernel": "mixed_batch call: reclaim + combining + lane kernel + what it hands on + combined results"},
             "cpu_baseline": cpu,
             "clocks": clk,
-            # reclaim, partition, find class, insert class, update combining,
-            # update/erase class, combined results: 7 kernels per step
-            "gpu_launches": 7 * args.steps,
+            # reclaim, update combining, one request per lane, what the lanes
+            # hand on, combined results: 5 kernels per step
+            "gpu_launches": 5 * args.steps,
             "pool": {"used_slabs": stats["used_slabs"], "total_slabs": stats["total_slabs"]},
         }
         res.update(extra)

@@ -5,7 +5,8 @@ Searches the form and launch shape of the call over
   sub-batches; or all sub-batches at once grouped by key) x
   find tile (lanes per find: 4, 8, 16, 32) x write tile (lanes per insert,
   update and erase: 16, 32) x key-length bucketing (off, on; the grouped
-  form has no buckets and runs once per tile pair),
+  form has no buckets and runs once per tile pair; the "forked" form serves one
+  request per lane and is the same at every tile and bucketing),
 then, for the best of those, blocks per SM 1..8.  This is coordinate descent
 (40 + 8 trials rather than the 384 points of the full grid): blocks per SM
 only trades occupancy against per-warp registers, and is measured with the
