@@ -814,6 +814,7 @@ MT_DEV void lane_serve(const tree_view& tv, const Src& src, const defer_list& dl
   const uint32_t per = max(1u, min(32u, (n + warps - 1u) / warps));
   slab_cache<32> cache;
   cache.init(p, warp);
+  cache.keeps = !TAIL;
 #pragma unroll 1
   for (uint32_t base = warp * per; base < n; base += warps * per) {
     if (__any_sync(kAll, slot == 0u && fatal_error(p))) break;

@@ -87,8 +87,11 @@ struct slab_cache {
   uint32_t slab = kInvalid;
   uint32_t count = 0;   // uniform over the tile
   uint32_t shard = 0;   // uniform: preferred shard
-  // Whole-warp tiles: slabs that a lane took and led nobody to, a list linked
-  // by their last words (mt_lane.cuh).  They are handed out first.
+  // Whole-warp tiles with `keeps` set: slabs that a lane took and led nobody to, a
+  // list linked by their last words (mt_lane.cuh).  They are handed out first.
+  // (A flag that a kernel never sets costs it nothing; without one, the vote on
+  // vain_n took 7% of the serving loop's peak.)
+  bool keeps = false;
   uint32_t vain = kInvalid;
   uint32_t vain_n = 0;
   // Set by kernels that follow one that gave slabs back unused: these are taken
@@ -146,7 +149,7 @@ struct slab_cache {
 
   // Returns a fresh slab index (uniform) or kInvalid after recording MT_ERR_OOM.
   MT_DEV uint32_t allocate(const tile<T>& t, const pool_view& p) {
-    if constexpr (T == 32) {
+    if (T == 32 && keeps) {
       const uint32_t m = t.ballot(vain_n != 0u);
       if (m) {
         const int l = __ffs(m) - 1;
@@ -222,7 +225,7 @@ MT_DEV void slab_cache<T>::release(const tile<T>& t, const pool_view& p) {
   if (t.rank < count && slab != kInvalid) retire_slab(p, slab);
   count = 0;
   slab = kInvalid;
-  if constexpr (T == 32) {
+  if (T == 32 && keeps) {
     for (; vain_n != 0u; --vain_n) {
       const uint32_t nx = ld_relaxed_u32(p.addr(vain) + kNextWord);
       retire_slab(p, vain);
